@@ -125,9 +125,10 @@ def _weights(gen, experts, rows, cols):
     return q, s
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """Layer weights, router logits and bias, bf16 activations."""
     gen = torch.Generator(device="cuda").manual_seed(seed)
-    tokens, experts, entry = case["tokens"], case["experts"], case["entry"]
+    tokens, experts = case["tokens"], case["experts"]
     w13, w13_scale = _weights(gen, experts, 2 * I, H)
     w2, w2_scale = _weights(gen, experts, H, I)
     bias, offsets = _router(case)
@@ -136,6 +137,12 @@ def prepare(case, seed):
     x = torch.randn((tokens, H), generator=gen, device="cuda").bfloat16()
     weights = {"gemm1_weights": w13, "gemm1_weights_scale": w13_scale, "gemm2_weights": w2,
                "gemm2_weights_scale": w2_scale}
+    return weights, logits, bias, x
+
+
+def prepare(case, seed):
+    tokens, entry = case["tokens"], case["entry"]
+    weights, logits, bias, x = _inputs(case, seed)
     state = {"entry": entry, "weights": weights, "offset": case["offset"], "logits": logits, "bias": bias}
     if entry == "bf16":
         state["x"] = x
@@ -163,6 +170,46 @@ def run(state):
         return {"hidden": hidden, "hidden_scale": hidden_scale, "out": out}
     return moe.kernel(state["logits"], state["bias"], state["hidden"], state["hidden_scale"],
                       local_expert_offset=state["offset"], routed_scaling_factor=SCALE, **state["weights"])
+
+
+def _route64(logits, bias):
+    """Group-limited top-8 in 64 bits: expert ids and weights."""
+    s = torch.sigmoid(logits.double())
+    by_group = (s + bias.double()).view(-1, GROUPS, EXPERTS // GROUPS)
+    keep = by_group.topk(2, dim=2).values.sum(dim=2).topk(TOP_GROUPS, dim=1).indices
+    mask = torch.zeros(by_group.shape[:2], device=logits.device).scatter_(1, keep, 1.0)
+    idx = torch.where(mask.unsqueeze(2) > 0, by_group, -1.0).view(-1, EXPERTS).topk(TOP_K, dim=1).indices
+    w = s.gather(1, idx)
+    return idx, w / (w.sum(dim=1, keepdim=True) + 1e-20) * SCALE
+
+
+def _dequant64(q, scale):
+    rows, cols = q.shape
+    return (q.double().view(rows // 128, 128, cols // 128, 128) * scale.double()[:, None, :, None]).view(rows, cols)
+
+
+def exact(case, seed):
+    """The layer in 64 bits on the same e4m3 values and scales."""
+    weights, logits, bias, x = _inputs(case, seed)
+    hidden, hidden_scale = _quantize_rows(x.double() if case["entry"] == "bf16" else x.float())
+    idx, w = _route64(logits, bias)
+    scale_rows = hidden_scale.t().double()
+    out = torch.zeros((case["tokens"], H), dtype=torch.float64, device="cuda")
+    for e in range(case["experts"]):
+        token, k = (idx == case["offset"] + e).nonzero(as_tuple=True)
+        if token.numel() == 0:
+            continue
+        w13 = _dequant64(weights["gemm1_weights"][e], weights["gemm1_weights_scale"][e])
+        w2 = _dequant64(weights["gemm2_weights"][e], weights["gemm2_weights_scale"][e])
+        for part in torch.arange(token.numel(), device="cuda").split(2048):
+            t = token[part]
+            a = (hidden[t].double().view(-1, H // 128, 128) * scale_rows[t].unsqueeze(2)).view(-1, H)
+            up, gate = (a @ w13.t()).split(I, dim=1)
+            y = (gate * torch.sigmoid(gate) * up) @ w2.t()
+            out.index_add_(0, t, y * w[t, k[part]].unsqueeze(1))
+    if case["entry"] == "bf16":
+        return {"hidden": None, "hidden_scale": hidden_scale, "out": out}
+    return out
 
 
 def work(case):
