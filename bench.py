@@ -621,7 +621,7 @@ def measure_workload(K, name, T_global, E1, skew, args, rank, world, device, pea
         # route, 3 x ranking, count exchange, pack, barrier, 7 x layer on the records, barrier, combine
         launches_per_step = 17
     elif _l.uses_decode_path(T_loc, E_local):
-        launches_per_step = 3          # route, GEMV1, GEMV2
+        launches_per_step = 2          # route + GEMV1, GEMV2
     elif T_loc <= _l.PROLOGUE_MAX_T:
         launches_per_step = 4          # fused prologue, GEMM1, GEMM2, reduce
     elif T_loc <= 1024:

@@ -27,6 +27,7 @@ int launch_gemm1_skinny(const b200moe_problem*, const b200moe_workspace*, int, c
 int launch_gemm2_skinny(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t, bool);
 int launch_reduce(const b200moe_problem*, const b200moe_workspace*, cudaStream_t, bool half_src);
 int launch_gemv1(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t);
+int launch_route_gemv1(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t);
 int launch_gemv2(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t);
 
 struct DeviceInfo {
@@ -367,12 +368,16 @@ int b200moe_forward(const b200moe_problem* p, const b200moe_workspace* ws, void*
   int sms;
   if ((rc = device_info(&sms))) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // Decode, at most eight tokens: every expert's tokens fit one N = 8 instruction and the whole batch's activations fit
+  // shared memory, so nothing has to be sorted or gathered and the weights go from HBM to the tensor core through
+  // registers.  Measured at the limit and below it (us per call, this path / the sorted path; E = local experts, skewed =
+  // hot experts that several tokens share): T = 8, E = 32 69 / 99, skewed 61 / 73; T = 8, E = 256 342 / 389, skewed
+  // 221 / 236; T = 8, E = 128 skewed 102 / 103; T = 1, E = 256 67 / 103; T = 6, E = 8 skewed 25 / 49.  Past eight tokens the
+  // f16 activations take the shared memory that the weight loads in flight need as L1 (T = 14, E = 32: 212 / 138).
   if (p->routing_logits && p->T <= B200MOE_DECODE_MAX_T && p->T * p->E_local <= B200MOE_DECODE_MAX_WORK &&
-      p->out_seg_count == 0 && !p->hidden_row_stride &&
+      p->out_seg_count == 0 && p->partial_format == B200MOE_PARTIAL_F32 && !p->hidden_row_stride &&
       !p->scale_token_stride && !p->scale_block_stride) {
-    // decode: a few tokens, one or two rows per expert — stream the weights through matrix-vector kernels
-    if ((rc = launch_route(p, ws, st))) return rc;
-    if ((rc = launch_gemv1(p, ws, sms, st))) return rc;
+    if ((rc = launch_route_gemv1(p, ws, sms, st))) return rc;
     return launch_gemv2(p, ws, sms, st);
   }
   bool after_gather = false;   // GEMM1 directly follows k_gather (whose release tells it the sort is complete)

@@ -1,21 +1,50 @@
-// Decode path (T <= B200MOE_DECODE_MAX_T tokens): the two expert matrices applied as matrix-vector products on the CUDA
-// cores, one warp per output element, weights streamed from HBM exactly once per (token, expert) pair.
+// Decode path (T <= B200MOE_DECODE_MAX_T tokens): two kernels, weights streamed from HBM once per expert that has a token.
 //
-// With a handful of tokens every expert sees one or two rows, a 128-row tensor-core tile is >98 % padding and — worse —
-// only (active experts x 16) CTAs have work, so the tile kernels pull a few hundred GB/s.  Here every SM streams
-// weights: 14 336 bytes of W13 per warp task in GEMV1 (rows n and 2048+n, fused SwiGLU), 2 048 bytes of W2 per expert in
-// GEMV2, which also applies the routing weights and sums the token's local experts, so the sort, the gather and the
-// reduce are not needed at all.  The intermediate is kept in fp32 and enters GEMV2 as f16 scaled by its row maximum.
+// With a handful of tokens every expert sees one or a few rows: a 128-row tile is padding, and the sort, the gather and
+// the tile pipeline of the larger paths cost more than the weights' journey from HBM.  Both kernels run one persistent
+// CTA per SM and keep the next pieces of weights in flight in registers (~110 KB per SM; HBM needs ~55).
+//
+//   k_gemv1_swiglu  (route, selection bits,) GEMM1 + SwiGLU.  Every CTA routes the whole batch by itself, a warp per token,
+//                   after the activations were put into shared memory as f16: no launch and no hand-over between routing
+//                   and the weight stream.  A task is eight intermediate columns of one expert as one
+//                     mma.sync m16n8k16, f16 x f16 -> f32 (e4m3 -> f16 is exact)
+//                   M rows 0..7 = W1 rows n.., M rows 8..15 = W3 rows 2048 + n.., N = the expert's tokens, so one thread
+//                   holds up and gate of the same (column, token).  K is permuted the same way on both sides: the 16
+//                   bytes a lane loads of a row are its A fragments, without a trip through shared memory.  Seven warps
+//                   take every seventh of the 56 K blocks of a task (a team reads 896 contiguous bytes per row at a time)
+//                   and add their sums through shared memory.
+//                   The instruction costs the same for one token and for eight, which is what it is for: packed half FMAs,
+//                   as in GEMV2, take 61 us instead of 26 for eight tokens on five hot experts (37 instead of 43 where
+//                   every expert has one token).  e4m3 mma.sync (m16n8k32) was slower: 40 us per call at T = 1 against 27.
+//   k_gemv2_reduce  GEMM2 and the weighted sum over experts on the CUDA cores.  A warp task is four output columns for the
+//                   whole batch: W2 rows in registers, the intermediate rows in shared memory as f16 scaled to |x| <= 7 by
+//                   their own maximum (11-bit rounding of each element, as the products'), packed half FMAs over 16 K
+//                   columns, fp32 from there on.  (The m16n8k16 form of it read 33 against 23 us at seven pairs.)
+//
+// Measured: see the dispatch rule in api.cu.
 // Reference counterpart: the T = 1 path, solution/python/pure_triton_impl.py:2025-2123 (_kernel_t1) with
 // _t1_fused_gemm2_reduce_kernel (:1676-1750); oracle math solution/cuda/binding.py:157-182.
+#include <cuda_fp16.h>
 #include "common.cuh"
+#include "gemm_common.cuh"
+#include "route_token.cuh"
 
 namespace b200moe {
 
-// Arithmetic: e4m3 -> f16 is exact, so 16-element partial dot products run on the packed half-precision FMA with the
-// activation pre-scaled by 2^-6 (|a| <= 7, |w| <= 448: eight products per lane sum to < 2^15, no overflow; each
-// product is rounded to 11 bits, far below the output tolerance) and are then added in fp32.  This needs 8 conversions
-// per 16 weights instead of 24 and is what keeps the kernels at the memory system's pace.
+constexpr int DEC_T = B200MOE_DECODE_MAX_T;
+constexpr int DEC_PAIRS = DEC_T * TOP_K;
+constexpr int DEC_N = 8;                                // tokens of one list = N of the instruction
+static_assert(DEC_T <= DEC_N, "an expert's tokens are one N tile, and one lane each in GEMV2's sums");
+
+// streaming 16-byte load: weights are read once, keep them out of L1
+__device__ __forceinline__ uint4 ld_stream(const uint8_t* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+// 16 e4m3 values -> f16, exactly.
 struct Half2x8 {
   __half2 v[8];
 };
@@ -31,219 +60,472 @@ __device__ __forceinline__ Half2x8 cvt16_h2(const uint4& q) {
   }
   return r;
 }
-__device__ __forceinline__ float dot16_h2(const Half2x8& a, const uint4& wq) {
-  const Half2x8 w = cvt16_h2(wq);
+__device__ __forceinline__ uint32_t half2_bits(const __half2& h) { return *reinterpret_cast<const uint32_t*>(&h); }
+// c += 64 K columns of 16 weight rows x 8 tokens.  lo / hi: the lane's 16 weights of M rows g and g + 8; b: the same 16 K
+// columns of token g (f16).  Four MMAs, each taking four of the lane's columns.
+__device__ __forceinline__ void mma_k64(float (&c)[4], const uint4& lo, const uint4& hi, const uint8_t* b) {
+  const Half2x8 x = cvt16_h2(lo), y = cvt16_h2(hi);
+  const uint4 b0 = reinterpret_cast<const uint4*>(b)[0], b1 = reinterpret_cast<const uint4*>(b)[1];
+  const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(half2_bits(x.v[2 * j])), "r"(half2_bits(y.v[2 * j])), "r"(half2_bits(x.v[2 * j + 1])),
+          "r"(half2_bits(y.v[2 * j + 1])), "r"(bw[2 * j]), "r"(bw[2 * j + 1]));
+}
+// Ask for bytes [p, p + bytes) to be brought into L2 (16-byte aligned, a multiple of 16; no completion to wait for).
+__device__ __forceinline__ void l2_prefetch_bulk(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// The batch seen expert by expert: lists of the tokens of each active local expert, experts ascending, tokens ascending.
+// Pair r of this order is row r of the intermediate.
+struct ExpertLists {
+  int n;                           // active experts
+  int warp_sum[E_GLOBAL / 32];
+  uint32_t mask[E_GLOBAL];         // bit t: token t selected the local expert
+  int e[DEC_PAIRS];
+  int first[DEC_PAIRS + 1];        // first pair of list u
+  uint8_t token[DEC_PAIRS];
+};
+
+// L.mask is complete (visible to the CTA).  Ends with a barrier.  The CTA has at least E_GLOBAL threads.
+__device__ __forceinline__ void build_lists(ExpertLists& L, int E_local) {
+  const int e = threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t mask = 0;
+  int incl = 0;
+  if (warp < E_GLOBAL / 32) {
+    mask = e < E_local ? L.mask[e] : 0u;
+    incl = (__popc(mask) << 16) | (mask != 0u);   // pairs and active experts in one scan
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += o;
+    }
+    if (lane == 31) L.warp_sum[warp] = incl;
+  }
+  __syncthreads();
+  if (warp < E_GLOBAL / 32) {
+    for (int w = 0; w < warp; ++w) incl += L.warp_sum[w];
+    if (mask) {
+      const int u = (incl & 0xffff) - 1;
+      int at = (incl >> 16) - __popc(mask);
+      L.e[u] = e;
+      L.first[u] = at;
+      for (uint32_t m = mask; m; m &= m - 1) L.token[at++] = static_cast<uint8_t>(__ffs(m) - 1);
+    }
+    if (threadIdx.x == E_GLOBAL - 1) {
+      L.n = incl & 0xffff;
+      L.first[incl & 0xffff] = incl >> 16;
+    }
+  }
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// GEMM1 + SwiGLU
+// ---------------------------------------------------------------------------------------------------------
+constexpr int G1_TEAM_WARPS = 7;                          // 56 K blocks, eight per warp
+constexpr int G1_TEAMS = 2;
+constexpr int G1_THREADS = G1_TEAMS * G1_TEAM_WARPS * 32; // 448: 144 registers per thread
+constexpr int G1_COLS = 8;
+constexpr int G1_ROW = 2 * H + 16;        // pitch of an activation row: tokens 16 bytes apart modulo 128, B loads without conflicts
+constexpr int G1_SCALES = H_BLOCKS + 1;
+constexpr int PART_PITCH = 20;        // floats per token of a partial sum: 16 rows + 4 (conflict-free stores)
+static_assert(G1_TEAM_WARPS * 8 == H_BLOCKS && G1_THREADS >= E_GLOBAL, "K split, list building");
+constexpr uint32_t W2_PREFETCH_BYTES = 32u << 20;         // about what HBM delivers while GEMV2 starts
+
+struct Gemv1Shared {
+  ExpertLists L;
+  float part[G1_TEAMS][G1_TEAM_WARPS][DEC_N * PART_PITCH];
+  float scale[DEC_T * G1_SCALES];     // activation scales, [token][K block]
+};
+static size_t gemv1_smem(int T) { return sizeof(Gemv1Shared) + 16 + static_cast<size_t>(T) * G1_ROW; }
+
+template <bool ROUTE>
+__global__ void __launch_bounds__(G1_THREADS, 1)
+k_gemv1_swiglu(const float* __restrict__ logits, const uint16_t* __restrict__ bias, float scale_factor,
+               int* __restrict__ topk_idx, float* __restrict__ topk_w, uint32_t* __restrict__ chunk_bits,
+               const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, int T, int local_offset,
+               int E_local, const uint8_t* __restrict__ w13, const float* __restrict__ w13_scale,
+               const uint8_t* __restrict__ w2, float* __restrict__ inter) {
+  extern __shared__ __align__(16) uint8_t dyn[];
+  uint8_t* rows = dyn;                                        // [T][G1_ROW]
+  Gemv1Shared& S = *reinterpret_cast<Gemv1Shared*>(dyn + static_cast<size_t>(T) * G1_ROW);
+  ExpertLists& L = S.L;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < E_GLOBAL) L.mask[threadIdx.x] = 0;
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int c = threadIdx.x; c < T * (H / 16); c += G1_THREADS) {
+    const int t = c / (H / 16), u = c - t * (H / 16);
+    const Half2x8 h = cvt16_h2(__ldg(reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(t) * H) + u));
+    uint4* dst = reinterpret_cast<uint4*>(rows + t * G1_ROW + u * 32);
+    dst[0] = *reinterpret_cast<const uint4*>(&h.v[0]);
+    dst[1] = *reinterpret_cast<const uint4*>(&h.v[4]);
+  }
+  for (int c = threadIdx.x; c < T * H_BLOCKS; c += G1_THREADS) {
+    const int kb = c / T, t = c - kb * T;
+    S.scale[t * G1_SCALES + kb] = __ldg(hidden_scale + c);
+  }
+  __syncthreads();   // masks are zero
+  for (int t = warp; t < T; t += G1_TEAMS * G1_TEAM_WARPS) {
+    int idx = 0;
+    if (ROUTE) {
+      float w;
+      route_token(logits + static_cast<size_t>(t) * E_GLOBAL, bias, scale_factor, lane, idx, w);
+      if (blockIdx.x == 0 && lane < TOP_K) {
+        topk_idx[t * TOP_K + lane] = idx;
+        topk_w[t * TOP_K + lane] = w;
+      }
+    } else if (lane < TOP_K) {
+      idx = topk_idx[t * TOP_K + lane];
+    }
+    const int le = idx - local_offset;
+    if (lane < TOP_K && le >= 0 && le < E_local) atomicOr(&L.mask[le], 1u << t);
+  }
+  __syncthreads();
+  if (ROUTE && blockIdx.x == 0 && threadIdx.x < E_local) chunk_bits[threadIdx.x] = L.mask[threadIdx.x];   // T <= 32: one chunk
+  build_lists(L, E_local);
+
+  const int team = warp / G1_TEAM_WARPS, wt = warp - team * G1_TEAM_WARPS;
+  const int tid_team = threadIdx.x - team * (G1_TEAM_WARPS * 32);
+  const int g = lane >> 2, q = lane & 3;
+  constexpr int TASKS_PER_LIST = I / G1_COLS;
+  const int n_teams = static_cast<int>(gridDim.x) * G1_TEAMS, my_team = blockIdx.x * G1_TEAMS + team;
+  const int tasks = L.n * TASKS_PER_LIST;
+  const int task_begin = tasks * my_team / n_teams, task_end = tasks * (my_team + 1) / n_teams;
+
+  // this lane's share of block kb of a task: 16 bytes at q * 16 and 64 + q * 16 of W1 row n + g and of W3 row n + g
+  auto task_ptr = [&](int task) {
+    const int u = task / TASKS_PER_LIST, n0 = (task - u * TASKS_PER_LIST) * G1_COLS;
+    return w13 + (static_cast<size_t>(L.e[u]) * 2 * I + n0 + g) * H + wt * 128 + q * 16;
+  };
+  // lanes 0..7: scales of W1 for the warp's eight blocks, lanes 8..15: of W3
+  auto task_scale = [&](int task) {
+    const int u = task / TASKS_PER_LIST, n0 = (task - u * TASKS_PER_LIST) * G1_COLS;
+    return __ldg(w13_scale + (static_cast<size_t>(L.e[u]) * 32 + (lane & 8) * 2 + (n0 >> 7)) * H_BLOCKS + (lane & 7) * G1_TEAM_WARPS + wt);
+  };
+  uint4 ring[4][4];
+  auto load = [&](uint4 (&s)[4], const uint8_t* p) {
+    s[0] = ld_stream(p);
+    s[1] = ld_stream(p + 64);
+    s[2] = ld_stream(p + static_cast<size_t>(I) * H);
+    s[3] = ld_stream(p + static_cast<size_t>(I) * H + 64);
+  };
+  const uint8_t* ptr = nullptr;
+  float wsc = 0.f;
+  if (task_begin < task_end) {
+    ptr = task_ptr(task_begin);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) load(ring[i], ptr + i * (G1_TEAM_WARPS * 128));
+    wsc = task_scale(task_begin);
+  }
+#pragma unroll 1
+  for (int task = task_begin; task < task_end; ++task) {
+    const int u = task / TASKS_PER_LIST, n0 = (task - u * TASKS_PER_LIST) * G1_COLS;
+    const int first = L.first[u], m = L.first[u + 1] - first;
+    const bool more = task + 1 < task_end;
+    const uint8_t* next = more ? task_ptr(task + 1) : ptr;
+    const float wsc_next = more ? task_scale(task + 1) : 0.f;
+    // columns past the list's last token repeat it; their sums are not used
+    const uint8_t* b_row = rows + L.token[first + min(g, m - 1)] * G1_ROW + wt * 256 + q * 32;
+    const float* x0 = S.scale + L.token[first + min(2 * q, m - 1)] * G1_SCALES + wt;
+    const float* x1 = S.scale + L.token[first + min(2 * q + 1, m - 1)] * G1_SCALES + wt;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      uint4 (&s)[4] = ring[i & 3];
+      const float w1 = __shfl_sync(0xffffffffu, wsc, i), w3 = __shfl_sync(0xffffffffu, wsc, 8 + i);
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+      mma_k64(c, s[0], s[2], b_row + i * (G1_TEAM_WARPS * 256));
+      mma_k64(c, s[1], s[3], b_row + i * (G1_TEAM_WARPS * 256) + 128);
+      acc[0] = fmaf(c[0], x0[i * G1_TEAM_WARPS] * w1, acc[0]);
+      acc[1] = fmaf(c[1], x1[i * G1_TEAM_WARPS] * w1, acc[1]);
+      acc[2] = fmaf(c[2], x0[i * G1_TEAM_WARPS] * w3, acc[2]);
+      acc[3] = fmaf(c[3], x1[i * G1_TEAM_WARPS] * w3, acc[3]);
+      if (i < 4) load(s, ptr + (i + 4) * (G1_TEAM_WARPS * 128));
+      else if (more) load(s, next + (i - 4) * (G1_TEAM_WARPS * 128));
+    }
+    float* a = S.part[team][wt] + 2 * q * PART_PITCH + g;
+    a[0] = acc[0];
+    a[PART_PITCH] = acc[1];
+    a[8] = acc[2];
+    a[PART_PITCH + 8] = acc[3];
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(G1_TEAM_WARPS * 32) : "memory");
+    if (tid_team < m * G1_COLS) {
+      const float* p = S.part[team][0] + (tid_team >> 3) * PART_PITCH + (tid_team & 7);
+      float up = 0.f, gate = 0.f;
+#pragma unroll
+      for (int w = 0; w < G1_TEAM_WARPS; ++w) {
+        up += p[w * (DEC_N * PART_PITCH)];
+        gate += p[w * (DEC_N * PART_PITCH) + 8];
+      }
+      inter[static_cast<size_t>(first + (tid_team >> 3)) * I + n0 + (tid_team & 7)] = gate / (1.0f + expf(-gate)) * up;
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(G1_TEAM_WARPS * 32) : "memory");
+    ptr = next;
+    wsc = wsc_next;
+  }
+  // GEMV2 reads W2 of the same experts: have its first rows on their way into L2 while the last columns finish here and
+  // the next kernel starts.
+  if (lane == 0 && L.n > 0 && w2) {
+    constexpr uint32_t PIECE = 8192, PER_EXPERT = static_cast<uint32_t>(H) * I / PIECE;
+    uint32_t per = W2_PREFETCH_BYTES / PIECE / static_cast<uint32_t>(L.n);
+    per = per < PER_EXPERT ? per : PER_EXPERT;
+    for (uint32_t i = blockIdx.x + gridDim.x * warp; i < per * L.n; i += gridDim.x * (G1_TEAMS * G1_TEAM_WARPS)) {
+      const uint32_t u = i / per;
+      l2_prefetch_bulk(w2 + static_cast<size_t>(L.e[u]) * H * I + static_cast<size_t>(i - u * per) * PIECE, PIECE);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// GEMM2 + weighted sum over experts
+// ---------------------------------------------------------------------------------------------------------
+// 16 K columns of one weight row (already f16) against one token's activations.
+__device__ __forceinline__ float dot16_h2(const Half2x8& a, const Half2x8& w) {
   __half2 acc = __hmul2(a.v[0], w.v[0]);
 #pragma unroll
   for (int i = 1; i < 8; ++i) acc = __hfma2(a.v[i], w.v[i], acc);
   const float2 f = __half22float2(acc);
   return f.x + f.y;
 }
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-  return v;
-}
-// streaming 16-byte load: weights are read once, keep them out of L1
-__device__ __forceinline__ uint4 ld_stream(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
+
+// Hides from the compiler that `w` is the same in every round of a loop.  Without it the f16 form of all weights a thread
+// holds is computed once before the loop over an expert's tokens (usually one): twice the registers, spilled.
+__device__ __forceinline__ void keep_packed(uint4& w) {
+  asm volatile("" : "+r"(w.x), "+r"(w.y), "+r"(w.z), "+r"(w.w));
 }
 
-constexpr int GEMV1_WARPS = 8;
-constexpr int GEMV1_N_PER_CTA = 8;    // one column pair (n, 2048 + n) per warp; 2048 / 8 = 256 CTAs per (token, expert)
-                                      // pair (measured at T = 1: 17.9 us against 21.3 us with 16 columns per CTA)
-constexpr int GEMV2_N_PER_CTA = 32;   // 7168 / 32 = 224 CTAs per token, 4 columns per warp (16 or 8 columns per CTA
-                                      // measured slower: every CTA stages the token's rows first)
+// The staged activation of token t (GEMV1): chunk c = 16 columns, two 16-byte units in swizzled order.
+__device__ __forceinline__ Half2x8 staged16(const uint4* row, int c) {
+  const int sw = (c >> 2) & 1;
+  Half2x8 a;
+  *reinterpret_cast<uint4*>(&a.v[0]) = row[2 * c + sw];
+  *reinterpret_cast<uint4*>(&a.v[4]) = row[2 * c + (sw ^ 1)];
+  return a;
+}
 
-// inter[p, n] = silu(x . W3[n]) * (x . W1[n]) for the local pair p = t*8+k of this CTA; the activation row is
-// converted once per CTA into shared memory (f16, pre-scaled by 2^-6), each warp then streams rows n and 2048+n.
-__global__ void __launch_bounds__(GEMV1_WARPS * 32)
-k_gemv1_swiglu(const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale,
-               const int* __restrict__ topk_idx, int T, int local_offset, int E_local,
-               const uint8_t* __restrict__ w13, const float* __restrict__ w13_scale, float* __restrict__ inter) {
-  __shared__ __align__(16) __half2 s_a[H / 2];   // 14 KB
-  __shared__ float s_as[H_BLOCKS];               // activation scales x 64
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int CTAS_PER_PAIR = I / GEMV1_N_PER_CTA;
-  const int p = blockIdx.x / CTAS_PER_PAIR;
-  const int n0 = (blockIdx.x - p * CTAS_PER_PAIR) * GEMV1_N_PER_CTA;
-  pdl_launch_dependents();
-  pdl_wait();
-  const int e = __ldg(topk_idx + p) - local_offset;
-  if (e < 0 || e >= E_local) return;
-  const int t = p / TOP_K;
-  {
-    const uint4* a_row = reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(t) * H);
-    const __half2 pre = __float2half2_rn(0.015625f);  // 2^-6, undone in s_as
-    for (int c = threadIdx.x; c < H / 16; c += blockDim.x) {
-      Half2x8 a = cvt16_h2(__ldg(a_row + c));
+constexpr int G2_WARPS = 16;
+constexpr int G2_THREADS = G2_WARPS * 32;
+constexpr int GEMV2_BATCH = 24;   // intermediate rows staged at a time (4 KB each)
+constexpr int GEMV2_COLS = 4;     // output columns per warp task
+
+// M intermediate rows (pairs q ..) of one expert against four rows of W2, converted to f16 once for all M; lane 8 c + t
+// adds column c of token t.
+template <int M>
+__device__ __forceinline__ void gemv2_rows(int q, int p0, int lane, const uint8_t* staged,
+                                           uint4 (&w)[GEMV2_COLS][I / 16 / 32], const float (&f)[I / 16 / 32],
+                                           const uint8_t* token, const float* s_back, float& tot) {
+  float acc[M][GEMV2_COLS];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s_a[c * 8 + j] = __hmul2(a.v[j], pre);
+  for (int r = 0; r < M; ++r)
+#pragma unroll
+    for (int j = 0; j < GEMV2_COLS; ++j) acc[r][j] = 0.f;
+#pragma unroll
+  for (int i = 0; i < I / 16 / 32; ++i) {
+    Half2x8 a[M];
+#pragma unroll
+    for (int r = 0; r < M; ++r)
+      a[r] = staged16(reinterpret_cast<const uint4*>(staged + static_cast<size_t>(q - p0 + r) * I * 2), i * 32 + lane);
+#pragma unroll
+    for (int j = 0; j < GEMV2_COLS; ++j) {
+      keep_packed(w[j][i]);
+      const Half2x8 h = cvt16_h2(w[j][i]);
+#pragma unroll
+      for (int r = 0; r < M; ++r) acc[r][j] = fmaf(dot16_h2(a[r], h), f[i], acc[r][j]);
     }
-    if (threadIdx.x < H_BLOCKS)
-      s_as[threadIdx.x] = 64.0f * __ldg(hidden_scale + static_cast<size_t>(threadIdx.x) * T + t);
   }
-  __syncthreads();
-  for (int n = n0 + warp; n < n0 + GEMV1_N_PER_CTA; n += GEMV1_WARPS) {
-    const uint4* w1_row = reinterpret_cast<const uint4*>(w13 + (static_cast<size_t>(e) * 2 * I + n) * H);
-    const uint4* w3_row = reinterpret_cast<const uint4*>(w13 + (static_cast<size_t>(e) * 2 * I + I + n) * H);
-    const float* s1 = w13_scale + (static_cast<size_t>(e) * 32 + (n >> 7)) * H_BLOCKS;
-    const float* s3 = w13_scale + (static_cast<size_t>(e) * 32 + 16 + (n >> 7)) * H_BLOCKS;
-    float acc1 = 0.f, acc3 = 0.f;
 #pragma unroll
-    for (int i = 0; i < H / 16 / 32; ++i) {
-      const int c = i * 32 + lane;       // 16-byte chunk of the row; 8 chunks per 128-column scale block
-      const int kb = c >> 3;
-      const uint4 wa = ld_stream(w1_row + c);
-      const uint4 wb = ld_stream(w3_row + c);
-      Half2x8 a;
-      const uint4* sa = reinterpret_cast<const uint4*>(s_a + c * 8);
-      *reinterpret_cast<uint4*>(&a.v[0]) = sa[0];
-      *reinterpret_cast<uint4*>(&a.v[4]) = sa[1];
-      const float as = s_as[kb];
-      acc1 = fmaf(dot16_h2(a, wa), as * __ldg(s1 + kb), acc1);
-      acc3 = fmaf(dot16_h2(a, wb), as * __ldg(s3 + kb), acc3);
-    }
-    acc1 = warp_sum(acc1);
-    acc3 = warp_sum(acc3);
-    if (lane == 0) inter[static_cast<size_t>(p) * I + n] = acc3 / (1.0f + expf(-acc3)) * acc1;
+  for (int r = 0; r < M; ++r) {
+    // four sums over 32 lanes; lanes 8 c .. 8 c + 7 end up with the sum of column c
+    const bool hi = (lane & 16) != 0, mid = (lane & 8) != 0;
+    float x0 = hi ? acc[r][2] : acc[r][0], x1 = hi ? acc[r][3] : acc[r][1];
+    x0 += __shfl_xor_sync(0xffffffffu, hi ? acc[r][0] : acc[r][2], 16);
+    x1 += __shfl_xor_sync(0xffffffffu, hi ? acc[r][1] : acc[r][3], 16);
+    float y = mid ? x1 : x0;
+    y += __shfl_xor_sync(0xffffffffu, mid ? x0 : x1, 8);
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) y += __shfl_xor_sync(0xffffffffu, y, d);
+    if ((lane & 7) == token[q + r]) tot = fmaf(s_back[q - p0 + r], y, tot);
   }
 }
 
-// out[t, n] = sum over the token's local experts of weight * (inter[p] . W2[e][n]).  One CTA = one token and 32
-// output columns; the token's (at most 8) intermediate rows are brought into shared memory once, as f16 scaled to
-// |x| <= 7 by the row's own maximum (11-bit rounding of each element; the dot products then run on packed half FMAs
-// like GEMV1).
-__global__ void __launch_bounds__(256)
+// out[t, n] = sum over the token's local experts of weight * (inter[p] . W2[e][n]).
+__global__ void __launch_bounds__(G2_THREADS, 1)
 k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx, const float* __restrict__ topk_w,
                int T, int local_offset, int E_local, const uint8_t* __restrict__ w2, const float* __restrict__ w2_scale,
                uint16_t* __restrict__ out, float* __restrict__ out_f32) {
-  __shared__ __align__(16) __half2 s_x[TOP_K][I / 2];   // 32 KB
-  __shared__ float s_back[TOP_K];                       // weight * row maximum / 7
-  __shared__ int s_e[TOP_K];
-  __shared__ float s_red[TOP_K][8];
+  extern __shared__ __align__(16) uint8_t dyn[];         // GEMV2_BATCH rows of 2048 f16
+  __shared__ float s_back[GEMV2_BATCH];                  // weight * row maximum / 7
+  __shared__ ExpertLists L;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int CTAS_PER_TOKEN = H / GEMV2_N_PER_CTA;
-  const int t = blockIdx.x / CTAS_PER_TOKEN;
-  const int n0 = (blockIdx.x - t * CTAS_PER_TOKEN) * GEMV2_N_PER_CTA;
+  const int G = gridDim.x;
+  if (threadIdx.x < E_GLOBAL) L.mask[threadIdx.x] = 0;
   pdl_launch_dependents();
   pdl_wait();
-  // Stage the token's local rows: all loads first (up to 8 rows x 8 floats per thread), one block-wide maximum for all
-  // rows at once, then the scaled f16 copies.  (Row by row this was a chain of 8 x (load, two barriers) before the first
-  // weight byte was requested.)
-  int e_k[TOP_K];
-  float4 v[TOP_K][2];
-  float m[TOP_K];
-#pragma unroll
-  for (int k = 0; k < TOP_K; ++k) {
-    const int p = t * TOP_K + k;
-    const int e = __ldg(topk_idx + p) - local_offset;
-    e_k[k] = (e >= 0 && e < E_local) ? e : -1;   // CTA-uniform
-    m[k] = 0.f;
-    if (e_k[k] >= 0) {
-      const float4* x = reinterpret_cast<const float4*>(inter + static_cast<size_t>(p) * I);
-#pragma unroll
-      for (int j = 0; j < 2; ++j) v[k][j] = __ldg(x + threadIdx.x * 2 + j);   // 256 threads x 8 floats = 2048
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < TOP_K; ++k) {
-    if (e_k[k] < 0) continue;
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-      m[k] = fmaxf(m[k], fmaxf(fmaxf(fabsf(v[k][j].x), fabsf(v[k][j].y)), fmaxf(fabsf(v[k][j].z), fabsf(v[k][j].w))));
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], d));
-    if (lane == 0) s_red[k][warp] = m[k];
-  }
-  if (threadIdx.x < TOP_K) s_e[threadIdx.x] = e_k[threadIdx.x];
   __syncthreads();
-#pragma unroll
-  for (int k = 0; k < TOP_K; ++k) {
-    if (e_k[k] < 0) continue;
-    float mk = s_red[k][0];
-#pragma unroll
-    for (int j = 1; j < 8; ++j) mk = fmaxf(mk, s_red[k][j]);
-    const float r = mk > 0.f ? 7.0f / mk : 0.f;
-    __half2* dst = &s_x[k][threadIdx.x * 4];
-    dst[0] = __floats2half2_rn(v[k][0].x * r, v[k][0].y * r);
-    dst[1] = __floats2half2_rn(v[k][0].z * r, v[k][0].w * r);
-    dst[2] = __floats2half2_rn(v[k][1].x * r, v[k][1].y * r);
-    dst[3] = __floats2half2_rn(v[k][1].z * r, v[k][1].w * r);
-    if (threadIdx.x == 0) s_back[k] = __ldg(topk_w + t * TOP_K + k) * mk * (1.0f / 7.0f);
+  if (threadIdx.x < T * TOP_K) {
+    const int le = __ldg(topk_idx + threadIdx.x) - local_offset;
+    if (le >= 0 && le < E_local) atomicOr(&L.mask[le], 1u << (threadIdx.x / TOP_K));
   }
   __syncthreads();
-  // Each warp owns 4 output columns (n0 + warp + 8 j).  Per local expert it first requests all 16 weight loads of its
-  // four rows (2 KB each), then consumes them: 8 KB in flight per warp instead of 2.
-  constexpr int COLS = GEMV2_N_PER_CTA / 8;
-  float total[COLS];   // per-lane shares; lanes are added once per column, after all of the token's experts
+  build_lists(L, E_local);
+  const int n_lists = L.n, n_pairs = L.first[L.n];
+
+  // Column groups of this CTA, one per warp and round.  A round keeps its sums while the batch's intermediate rows pass
+  // through shared memory GEMV2_BATCH at a time (one pass unless the batch has more pairs than that).
+  constexpr int GROUPS = H / GEMV2_COLS;
+  const int g_begin = GROUPS * blockIdx.x / G, g_end = GROUPS * (blockIdx.x + 1) / G;
+  const bool vec_store = ((reinterpret_cast<uintptr_t>(out) & 7u) | (reinterpret_cast<uintptr_t>(out_f32) & 15u)) == 0;
+  int staged = -1;   // first pair of the rows in shared memory
+  for (int g0 = g_begin; g0 < g_end; g0 += G2_WARPS) {
+    const int g = g0 + warp;
+    const int n0 = g * GEMV2_COLS;
+    float tot = 0.f;   // lane 8 c + t: column n0 + c of token t
+    int u = 0;
+    for (int p0 = 0; p0 < n_pairs; p0 += GEMV2_BATCH) {
+      const int p1 = p0 + GEMV2_BATCH < n_pairs ? p0 + GEMV2_BATCH : n_pairs;
+      if (staged != p0) {
+        if (staged >= 0) __syncthreads();   // everybody has finished with the rows that are replaced
+        // one warp per row: f16 scaled to |x| <= 7 by the row's own maximum (11-bit rounding of each element)
+#pragma unroll 1
+        for (int r = warp; r < p1 - p0; r += G2_WARPS) {
+          const float4* x = reinterpret_cast<const float4*>(inter + static_cast<size_t>(p0 + r) * I);
+          float4 v[I / 4 / 32];
+          float m = 0.f;
 #pragma unroll
-  for (int j = 0; j < COLS; ++j) total[j] = 0.f;
-  for (int k = 0; k < TOP_K; ++k) {
-    const int e = s_e[k];
-    if (e < 0) continue;
-    const float* sc = w2_scale + (static_cast<size_t>(e) * H_BLOCKS + (n0 >> 7)) * I_BLOCKS;
-    uint4 w[COLS][I / 16 / 32];
+          for (int i = 0; i < I / 16 / 32; ++i)
 #pragma unroll
-    for (int j = 0; j < COLS; ++j) {
-      const uint4* w_row = reinterpret_cast<const uint4*>(w2 + (static_cast<size_t>(e) * H + n0 + warp + 8 * j) * I);
+            for (int q = 0; q < 4; ++q) v[4 * i + q] = __ldg(x + (i * 32 + lane) * 4 + q);
 #pragma unroll
-      for (int i = 0; i < I / 16 / 32; ++i) w[j][i] = ld_stream(w_row + i * 32 + lane);
-    }
-    float acc[COLS];
+          for (int i = 0; i < I / 4 / 32; ++i)
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
 #pragma unroll
-    for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
+          for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+          const float k = m > 0.f ? 7.0f / m : 0.f;
+          uint4* dst = reinterpret_cast<uint4*>(dyn + static_cast<size_t>(r) * I * 2);
 #pragma unroll
-    for (int i = 0; i < I / 16 / 32; ++i) {
-      const int c = i * 32 + lane;
-      Half2x8 a;
-      const uint4* sa = reinterpret_cast<const uint4*>(&s_x[k][c * 8]);
-      *reinterpret_cast<uint4*>(&a.v[0]) = sa[0];
-      *reinterpret_cast<uint4*>(&a.v[4]) = sa[1];
-      const float scale = __ldg(sc + (c >> 3));
+          for (int i = 0; i < I / 16 / 32; ++i) {
+            Half2x8 a;
 #pragma unroll
-      for (int j = 0; j < COLS; ++j) acc[j] = fmaf(dot16_h2(a, w[j][i]), scale, acc[j]);
-    }
-    const float back = s_back[k];
-#pragma unroll
-    for (int j = 0; j < COLS; ++j) total[j] = fmaf(back, acc[j], total[j]);
-  }
-#pragma unroll
-  for (int j = 0; j < COLS; ++j) {
-    const float sum = warp_sum(total[j]);
-    const int n = n0 + warp + 8 * j;
-    if (lane == 0) {
-      if (out) {
-        __nv_bfloat16 b = __float2bfloat16_rn(sum);
-        out[static_cast<size_t>(t) * H + n] = *reinterpret_cast<uint16_t*>(&b);
+            for (int q = 0; q < 4; ++q) {
+              a.v[2 * q] = __floats2half2_rn(v[4 * i + q].x * k, v[4 * i + q].y * k);
+              a.v[2 * q + 1] = __floats2half2_rn(v[4 * i + q].z * k, v[4 * i + q].w * k);
+            }
+            const int c = i * 32 + lane, sw = (c >> 2) & 1;
+            dst[2 * c + sw] = *reinterpret_cast<const uint4*>(&a.v[0]);
+            dst[2 * c + (sw ^ 1)] = *reinterpret_cast<const uint4*>(&a.v[4]);
+          }
+          // the slot k in which the pair's token holds the pair's expert
+          int u_r = 0;
+          while (L.first[u_r + 1] <= p0 + r) ++u_r;
+          const int t = L.token[p0 + r];
+          const bool hit = lane < TOP_K && __ldg(topk_idx + t * TOP_K + lane) == L.e[u_r] + local_offset;
+          if (hit) s_back[r] = __ldg(topk_w + t * TOP_K + lane) * m * (1.0f / 7.0f);
+        }
+        staged = p0;
+        __syncthreads();
       }
-      if (out_f32) out_f32[static_cast<size_t>(t) * H + n] = sum;
+      if (g >= g_end) continue;
+      while (u < n_lists && L.first[u] < p1) {
+        const int e = L.e[u];
+        const uint4* w_row = reinterpret_cast<const uint4*>(w2 + (static_cast<size_t>(e) * H + n0) * I) + lane;
+        const float* sc = w2_scale + (static_cast<size_t>(e) * H_BLOCKS + (n0 >> 7)) * I_BLOCKS + (lane >> 3);
+        uint4 w[GEMV2_COLS][I / 16 / 32];
+        float f[I / 16 / 32];
+#pragma unroll
+        for (int j = 0; j < GEMV2_COLS; ++j)
+#pragma unroll
+          for (int i = 0; i < I / 16 / 32; ++i) w[j][i] = ld_stream(reinterpret_cast<const uint8_t*>(w_row + j * (I / 16) + i * 32));
+#pragma unroll
+        for (int i = 0; i < I / 16 / 32; ++i) f[i] = __ldg(sc + 4 * i);
+        const int first = L.first[u], last = L.first[u + 1];
+        const int q1 = last < p1 ? last : p1;
+        int q = first > p0 ? first : p0;
+#pragma unroll 1
+        for (; q + 1 < q1; q += 2) gemv2_rows<2>(q, p0, lane, dyn, w, f, L.token, s_back, tot);
+        if (q < q1) gemv2_rows<1>(q, p0, lane, dyn, w, f, L.token, s_back, tot);
+        if (last > p1) break;   // the rest of this expert's tokens are in the next batch of rows
+        ++u;
+      }
+    }
+    const float c1 = __shfl_down_sync(0xffffffffu, tot, 8), c2 = __shfl_down_sync(0xffffffffu, tot, 16),
+                c3 = __shfl_down_sync(0xffffffffu, tot, 24);
+    if (g < g_end && lane < T) {
+      const float v[GEMV2_COLS] = {tot, c1, c2, c3};
+      const size_t at = static_cast<size_t>(lane) * H + n0;
+      if (out) {
+        uint16_t b[GEMV2_COLS];
+#pragma unroll
+        for (int j = 0; j < GEMV2_COLS; ++j) {
+          const __nv_bfloat16 x = __float2bfloat16_rn(v[j]);
+          b[j] = *reinterpret_cast<const uint16_t*>(&x);
+        }
+        if (vec_store) {
+          *reinterpret_cast<uint2*>(out + at) = make_uint2(b[0] | (static_cast<uint32_t>(b[1]) << 16),
+                                                           b[2] | (static_cast<uint32_t>(b[3]) << 16));
+        } else {
+#pragma unroll
+          for (int j = 0; j < GEMV2_COLS; ++j) out[at + j] = b[j];
+        }
+      }
+      if (out_f32) {
+        if (vec_store) {
+          *reinterpret_cast<float4*>(out_f32 + at) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < GEMV2_COLS; ++j) out_f32[at + j] = v[j];
+        }
+      }
     }
   }
 }
 
-// `inter` lives in the workspace's expert_out array (unused by this path): [T*8, 2048] floats.
-int launch_gemv1(const b200moe_problem* p, const b200moe_workspace* ws, int num_sms, cudaStream_t st) {
+// `inter` lives in the workspace's expert_out array (unused by this path): one row of 2048 floats per local pair.
+template <bool ROUTE>
+static int launch_gemv1_as(const b200moe_problem* p, const b200moe_workspace* ws, int num_sms, cudaStream_t st) {
   if (p->T == 0) return B200MOE_OK;
-  (void)num_sms;
-  const unsigned grid = static_cast<unsigned>(p->T) * TOP_K * (I / GEMV1_N_PER_CTA);
-  B200MOE_CUDA_TRY(launch_pdl(k_gemv1_swiglu, dim3(grid), dim3(GEMV1_WARPS * 32), 0, st, p->hidden_states,
-                              p->hidden_states_scale, ws->topk_idx, p->T, p->local_expert_offset, p->E_local,
-                              p->gemm1_weights, p->gemm1_weights_scale, ws->expert_out));
+  static bool attr_set[64] = {};
+  int dev = 0;
+  B200MOE_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 64 && !attr_set[dev]) {
+    B200MOE_CUDA_TRY(cudaFuncSetAttribute(k_gemv1_swiglu<ROUTE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(gemv1_smem(DEC_T))));
+    attr_set[dev] = true;
+  }
+  B200MOE_CUDA_TRY(launch_pdl(k_gemv1_swiglu<ROUTE>, dim3(num_sms), dim3(G1_THREADS), gemv1_smem(p->T), st,
+                              p->routing_logits, p->routing_bias, p->routed_scaling_factor, ws->topk_idx, ws->topk_w,
+                              ws->chunk_bits, p->hidden_states, p->hidden_states_scale, p->T, p->local_expert_offset,
+                              p->E_local, p->gemm1_weights, p->gemm1_weights_scale,
+                              ROUTE ? p->gemm2_weights : nullptr, ws->expert_out));   // the stage call leaves W2 alone
   return B200MOE_OK;
+}
+int launch_gemv1(const b200moe_problem* p, const b200moe_workspace* ws, int num_sms, cudaStream_t st) {
+  return launch_gemv1_as<false>(p, ws, num_sms, st);
+}
+// routing, selection bits and GEMV1 in one launch
+int launch_route_gemv1(const b200moe_problem* p, const b200moe_workspace* ws, int num_sms, cudaStream_t st) {
+  return launch_gemv1_as<true>(p, ws, num_sms, st);
 }
 
 int launch_gemv2(const b200moe_problem* p, const b200moe_workspace* ws, int num_sms, cudaStream_t st) {
   if (p->T == 0) return B200MOE_OK;
-  (void)num_sms;
-  const unsigned grid = static_cast<unsigned>(p->T) * (H / GEMV2_N_PER_CTA);
-  B200MOE_CUDA_TRY(launch_pdl(k_gemv2_reduce, dim3(grid), dim3(256), 0, st, ws->expert_out, ws->topk_idx, ws->topk_w,
-                              p->T, p->local_expert_offset, p->E_local, p->gemm2_weights, p->gemm2_weights_scale,
-                              p->output, p->output_f32));
+  static bool attr_set[64] = {};
+  int dev = 0;
+  constexpr int SMEM = GEMV2_BATCH * I * 2;
+  B200MOE_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 64 && !attr_set[dev]) {
+    B200MOE_CUDA_TRY(cudaFuncSetAttribute(k_gemv2_reduce, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          SMEM));
+    attr_set[dev] = true;
+  }
+  B200MOE_CUDA_TRY(launch_pdl(k_gemv2_reduce, dim3(num_sms), dim3(G2_THREADS), SMEM, st, ws->expert_out,
+                              ws->topk_idx, ws->topk_w, p->T, p->local_expert_offset, p->E_local, p->gemm2_weights,
+                              p->gemm2_weights_scale, p->output, p->output_f32));
   return B200MOE_OK;
 }
 

@@ -43,7 +43,7 @@ extern "C" {
 #define B200MOE_PROLOGUE_MAX_T 32  /* largest batch of b200moe_prologue_small */
 #define B200MOE_DECODE_MAX_T 8 /* the matrix-vector (decode) stages take at most this many tokens; b200moe_forward
                                   uses them while T * E_local <= B200MOE_DECODE_MAX_WORK */
-#define B200MOE_DECODE_MAX_WORK 128 /* = 4 expected (token, local expert) pairs: T * 8 * E_local / 256 */
+#define B200MOE_DECODE_MAX_WORK 2048 /* every number of local experts: eight tokens x 256 */
 
 enum {
   B200MOE_OK = 0,
@@ -184,7 +184,8 @@ int b200moe_workspace_init(const b200moe_workspace* ws /* host */, void* stream)
 
 /* Whole layer: route -> rank -> scatter -> gather -> GEMM1+SwiGLU -> GEMM2 -> weighted reduce, all on `stream`,
  * no host synchronisation.  With routing_logits given, T <= B200MOE_DECODE_MAX_T and T * E_local <=
- * B200MOE_DECODE_MAX_WORK it runs route -> GEMV1+SwiGLU -> GEMV2+reduce instead (b200moe_gemv1 / b200moe_gemv2 below): no sort, no gather, fp32 intermediate.  Replaces solution/python/pure_triton_impl.py:2125-2403 (kernel), :2025-2123 (_kernel_t1),
+ * B200MOE_DECODE_MAX_WORK it runs (route + GEMV1 + SwiGLU) -> (GEMV2 + reduce) instead, two launches with the results of
+ * b200moe_route, b200moe_gemv1, b200moe_gemv2 below: no sort, no gather, fp32 intermediate.  Replaces solution/python/pure_triton_impl.py:2125-2403 (kernel), :2025-2123 (_kernel_t1),
  * solution/python/triton_impl.py:346-566 and solution/python/triton_impl_t901.py:40-185. */
 int b200moe_forward(const b200moe_problem* p /* host */, const b200moe_workspace* ws /* host */, void* stream);
 
@@ -237,7 +238,7 @@ int b200moe_gemm2(const b200moe_problem* p, const b200moe_workspace* ws, void* s
 int b200moe_gemm1_skinny(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);
 int b200moe_gemm2_skinny(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);
 /* Decode path stages (need topk_idx / topk_w of b200moe_route in the workspace; the fp32 intermediate [T*8, 2048] is
- * kept in the workspace's expert_out array): one warp per output element streams the weight rows from HBM.
+ * kept in the workspace's expert_out array, one row per local pair, experts ascending, tokens ascending within one).
  * Replaces the reference's T = 1 path: GEMM1 with BLOCK_M = 16 (solution/python/pure_triton_impl.py:1824-1940) and
  * _t1_fused_gemm2_reduce_kernel (solution/python/pure_triton_impl.py:1676-1750). */
 int b200moe_gemv1(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);

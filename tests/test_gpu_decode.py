@@ -1,0 +1,50 @@
+"""GPU: the decode path (at most eight tokens) where its work split changes: one expert for all tokens, more pairs than one
+staging pass of the second kernel holds, every token on experts of its own, no local expert for some tokens; against the CPU
+oracle, and the stage entry points against the whole call."""
+import ctypes as C
+
+import pytest
+import torch
+
+from test_gpu_parity import gpu_inputs, moe, run_and_check  # noqa: F401  (fixture and helpers)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,E_local,seed,offset,skew", [
+    (8, 256, 31, 0, False),    # 64 pairs: three staging passes, a list cut between two of them
+    (8, 256, 32, 0, True),     # 64 pairs on few experts: lists of several tokens
+    (5, 256, 33, 0, True),     # 40 pairs
+    (3, 256, 34, 0, False),    # exactly 24 pairs: one full staging pass
+    (8, 32, 35, 32, True),     # hot experts
+    (7, 5, 36, 201, True),     # fewer experts than tokens, tokens without a local expert
+    (8, 1, 37, 77, True),      # one expert
+    (2, 128, 38, 128, False),
+])
+def test_decode_matches_oracle(moe, oracle, T, E_local, seed, offset, skew):  # noqa: F811
+    out, ref, _ = run_and_check(moe, oracle, T, E_local, seed, offset, skew)
+    empty = (torch.as_tensor(ref["out_bf16"]).float() == 0).all(dim=1)
+    assert not out.cpu()[empty].any()
+
+
+@pytest.mark.parametrize("T,E_local,skew", [(1, 32, False), (8, 256, True), (6, 32, True)])
+def test_decode_stages_equal_the_call(moe, T, E_local, skew):  # noqa: F811
+    """route, gemv1, gemv2 launched one by one give the bytes of the whole call (which routes inside gemv1), into bf16 and
+    into float32, also where the destination is aligned to its element only."""
+    from fused_moe_b200 import _lib
+    from fused_moe_b200.kernel import _problem
+    lib = _lib.load()
+    inp = gpu_inputs(T, E_local, 41, 0, skew)
+    whole = moe.kernel(**inp)
+    ws = moe.last_workspace()
+    stream = torch.cuda.current_stream().cuda_stream
+    flat16 = torch.full((T * 7168 + 1,), 3.0, dtype=torch.bfloat16, device="cuda")
+    flat32 = torch.full((T * 7168 + 1,), 3.0, dtype=torch.float32, device="cuda")
+    for out in (flat16[:-1], flat16[1:], flat32[:-1], flat32[1:]):
+        p = _problem(T, E_local, 0, float(inp["routed_scaling_factor"]), inp["routing_logits"], inp["routing_bias"],
+                     inp["hidden_states"], inp["hidden_states_scale"], inp["gemm1_weights"], inp["gemm1_weights_scale"],
+                     inp["gemm2_weights"], inp["gemm2_weights_scale"], out)
+        for stage in ("route", "gemv1", "gemv2"):
+            _lib.check(getattr(lib, "b200moe_" + stage)(C.byref(p), C.byref(ws.struct), stream), stage)
+        torch.cuda.synchronize()
+        assert torch.equal(out.view(T, 7168).to(torch.bfloat16), whole)
