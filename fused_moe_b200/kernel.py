@@ -100,14 +100,14 @@ def _workspace(device: torch.device, T: int, E_local: int, stream_ptr: int) -> _
         st.mirror = torch.zeros(4, dtype=torch.int32).pin_memory()
         st.mirror_np = st.mirror.numpy()
     _raise_if_failed(st)
-    need = workspace_bytes(T, E_local)
-    if st.buffer is None or st.buffer.numel() < need:
-        st.buffer = torch.empty(need, dtype=torch.uint8, device=device)
-        st.carved.clear()
-        st.active = None
     key = (T, E_local)
     ws = st.carved.get(key)
     if ws is None:
+        need = workspace_bytes(T, E_local)
+        if st.buffer is None or st.buffer.numel() < need:
+            st.buffer = torch.empty(need, dtype=torch.uint8, device=device)
+            st.carved.clear()
+            st.active = None
         s = _lib.Workspace()
         base = st.buffer.data_ptr()
         _lib.check(lib.b200moe_workspace_carve(base, st.buffer.numel(), T, E_local, C.byref(s)),
@@ -125,13 +125,13 @@ def _workspace(device: torch.device, T: int, E_local: int, stream_ptr: int) -> _
 
 
 def _require(t: torch.Tensor, name: str, dtype: torch.dtype, shape: Tuple[int, ...]) -> torch.Tensor:
-    if not torch.is_tensor(t):
+    if not isinstance(t, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
-    if t.dtype != dtype:
+    if t.dtype is not dtype:
         raise TypeError(f"{name} must be {dtype}, got {t.dtype}")
-    if tuple(t.shape) != shape:
+    if t.shape != shape:
         raise ValueError(f"{name} must have shape {shape}, got {tuple(t.shape)}")
-    return t if t.is_contiguous() else t.contiguous()
+    return t if t.is_contiguous() else t.detach().contiguous()
 
 
 def _require_cuda(**tensors) -> None:
@@ -176,9 +176,11 @@ def _check_weights(hidden_states, gemm1_weights, gemm1_weights_scale, gemm2_weig
 
 def _run(T, E_local, offset, scale, logits, bias, hs, hs_scale, w13, w13s, w2, w2s, output, topk_idx, topk_w,
          out_dtype=torch.bfloat16):
-    _require_cuda(routing_logits=logits, routing_bias=bias, hidden_states=hs, hidden_states_scale=hs_scale,
-                  gemm1_weights=w13, gemm1_weights_scale=w13s, gemm2_weights=w2, gemm2_weights_scale=w2s,
-                  topk_idx=topk_idx, topk_weights=topk_w)
+    for t in (logits, bias, hs, hs_scale, w13, w13s, w2, w2s, topk_idx, topk_w):
+        if t is not None and not t.is_cuda:
+            _require_cuda(routing_logits=logits, routing_bias=bias, hidden_states=hs, hidden_states_scale=hs_scale,
+                          gemm1_weights=w13, gemm1_weights_scale=w13s, gemm2_weights=w2, gemm2_weights_scale=w2s,
+                          topk_idx=topk_idx, topk_weights=topk_w)
     device = hs.device
     if offset < 0 or offset + E_local > E_GLOBAL:
         raise ValueError(f"local_expert_offset {offset} with {E_local} local experts exceeds {E_GLOBAL} experts")
@@ -191,18 +193,25 @@ def _run(T, E_local, offset, scale, logits, bias, hs, hs_scale, w13, w13s, w2, w
             raise RuntimeError("output must live on the device of hidden_states")
     if T == 0:
         return output
-    with torch.cuda.device(device):
-        stream_ptr = torch.cuda.current_stream(device).cuda_stream
-        ws = _workspace(device, T, E_local, stream_ptr)
-        p = _problem(T, E_local, offset, scale, logits, bias, hs, hs_scale, w13, w13s, w2, w2s, output, topk_idx,
-                     topk_w)
-        _lib.check(_lib.load().b200moe_forward(C.byref(p), C.byref(ws.struct), stream_ptr), "b200moe_forward")
-        if os.environ.get("B200MOE_CHECK_STATUS") == "1":
-            check_status(device)
+    if torch.cuda.current_device() == device.index:   # the usual case: no context manager on the way to the launch
+        _launch(device, T, E_local, offset, scale, logits, bias, hs, hs_scale, w13, w13s, w2, w2s, output, topk_idx, topk_w)
+    else:
+        with torch.cuda.device(device):
+            _launch(device, T, E_local, offset, scale, logits, bias, hs, hs_scale, w13, w13s, w2, w2s, output, topk_idx,
+                    topk_w)
     return output
 
 
-@torch.no_grad()
+def _launch(device, T, E_local, offset, scale, logits, bias, hs, hs_scale, w13, w13s, w2, w2s, output, topk_idx, topk_w):
+    """One layer call on the current stream of `device`, which is the current device."""
+    stream_ptr = torch.cuda.current_stream(device).cuda_stream
+    ws = _workspace(device, T, E_local, stream_ptr)
+    p = _problem(T, E_local, offset, scale, logits, bias, hs, hs_scale, w13, w13s, w2, w2s, output, topk_idx, topk_w)
+    _lib.check(_lib.load().b200moe_forward(C.byref(p), C.byref(ws.struct), stream_ptr), "b200moe_forward")
+    if os.environ.get("B200MOE_CHECK_STATUS") == "1":
+        check_status(device)
+
+
 def kernel(
     routing_logits,
     routing_bias,
