@@ -160,13 +160,18 @@ k_scatter(const int* __restrict__ topk_idx, const float* __restrict__ topk_w, lo
 }
 
 // Copy the e4m3 row and the 56 scales of each real sorted row; pad rows are left as they are (their products are
-// never read).  One warp per row, grid-stride over the rows that exist.
+// never read).  The first `row_ctas` CTAs copy rows, one warp per row, grid-stride over the rows that exist.  The others
+// copy scales: a warp takes 32 consecutive sorted rows, a lane each, and seven of the 56 scale blocks, so that
+// a_scale_sorted ([block][row]) is written 128 contiguous bytes at a time.  (With the row's own warp writing its 56 scales,
+// 4 bytes at a stride of 4 R_max, the kernel took 345 us for 131072 rows, now 319; 1500 tokens / 64 experts 11.3 -> 9.0 us,
+// 333 tokens / 32 experts 5.2 -> 4.3 us.)
 __global__ void __launch_bounds__(256)
 k_gather(const uint8_t* __restrict__ hidden, long long row_stride, const float* __restrict__ hidden_scale,
          long long scale_token_stride, long long scale_block_stride, int T,
-         const int* __restrict__ sorted_token_ids, const int* __restrict__ total_blocks, int R_max,
+         const int* __restrict__ sorted_token_ids, const int* __restrict__ total_blocks, int R_max, int row_ctas,
          uint8_t* __restrict__ a_sorted, float* __restrict__ a_scale_sorted) {
   const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
   const int warps_per_cta = blockDim.x >> 5;
   // Dependents are released only AFTER this kernel's own dependency wait: a GEMM1 that starts because of this release
   // may then read the sort metadata (complete, since every CTA here has seen the scatter finish) and stream its first
@@ -174,16 +179,28 @@ k_gather(const uint8_t* __restrict__ hidden, long long row_stride, const float* 
   pdl_wait();
   pdl_launch_dependents();
   const int rows = __ldg(total_blocks) * BLOCK_M;
-  for (int r = blockIdx.x * warps_per_cta + (threadIdx.x >> 5); r < rows; r += gridDim.x * warps_per_cta) {
-    int tok = __ldg(sorted_token_ids + r);
+  if (static_cast<int>(blockIdx.x) >= row_ctas) {
+    constexpr int PER = H_BLOCKS / 8;   // scale blocks of a warp: the eight warps of a CTA share 32 rows
+    for (int r0 = (blockIdx.x - row_ctas) * 32; r0 < rows; r0 += (gridDim.x - row_ctas) * 32) {
+      const int tok = __ldg(sorted_token_ids + r0 + lane);
+      if (tok >= T) continue;
+      const float* src = hidden_scale + static_cast<size_t>(tok) * scale_token_stride +
+                         static_cast<size_t>(warp * PER) * scale_block_stride;
+      float v[PER];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) v[i] = __ldg(src + static_cast<size_t>(i) * scale_block_stride);
+#pragma unroll
+      for (int i = 0; i < PER; ++i) a_scale_sorted[static_cast<size_t>(warp * PER + i) * R_max + r0 + lane] = v[i];
+    }
+    return;
+  }
+  for (int r = blockIdx.x * warps_per_cta + warp; r < rows; r += row_ctas * warps_per_cta) {
+    const int tok = __ldg(sorted_token_ids + r);
     if (tok >= T) continue;
     const uint4* src = reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(tok) * row_stride);
     uint4* dst = reinterpret_cast<uint4*>(a_sorted + static_cast<size_t>(r) * H);
 #pragma unroll
     for (int i = 0; i < H / 16 / 32; ++i) dst[i * 32 + lane] = __ldg(src + i * 32 + lane);
-    for (int kb = lane; kb < H_BLOCKS; kb += 32)
-      a_scale_sorted[static_cast<size_t>(kb) * R_max + r] =
-          __ldg(hidden_scale + static_cast<size_t>(kb) * scale_block_stride + static_cast<size_t>(tok) * scale_token_stride);
   }
 }
 
@@ -472,11 +489,13 @@ int launch_gather(const b200moe_problem* p, const b200moe_workspace* ws, int num
   int grid = static_cast<int>((max_rows + 7) / 8);
   if (grid > num_sms * 8) grid = num_sms * 8;
   if (grid < 1) grid = 1;
-  B200MOE_CUDA_TRY(launch_pdl(k_gather, dim3(grid), dim3(256), 0, st, p->hidden_states,
+  const int scale_ctas = static_cast<int>(max_rows / 32 < num_sms ? max_rows / 32 : num_sms);
+  B200MOE_CUDA_TRY(launch_pdl(k_gather, dim3(grid + scale_ctas), dim3(256), 0, st, p->hidden_states,
                               p->hidden_row_stride ? p->hidden_row_stride : static_cast<long long>(H),
                               p->hidden_states_scale, p->scale_token_stride ? p->scale_token_stride : 1LL,
                               p->scale_block_stride ? p->scale_block_stride : static_cast<long long>(p->T), p->T,
-                              ws->sorted_token_ids, ws->total_blocks, ws->R_max, ws->a_sorted, ws->a_scale_sorted));
+                              ws->sorted_token_ids, ws->total_blocks, ws->R_max, grid, ws->a_sorted,
+                              ws->a_scale_sorted));
   return B200MOE_OK;
 }
 
