@@ -20,8 +20,8 @@ int launch_route_topk(const float*, const uint16_t*, int, float, int*, float*, c
 int launch_small_prologue(const b200moe_problem*, const b200moe_workspace*, cudaStream_t);
 int launch_sort(const b200moe_problem*, const b200moe_workspace*, cudaStream_t);
 int launch_gather(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t);
-int launch_gemm1(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t);
-int launch_gemm2(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t, bool half_out);
+int launch_gemm1(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t, bool behind_gather);
+int launch_gemm2(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t, bool half_out, bool behind_gemm1);
 int launch_quantize_act(const void*, int, void*, float*, int, cudaStream_t);
 int launch_gemm1_skinny(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t, bool);
 int launch_gemm2_skinny(const b200moe_problem*, const b200moe_workspace*, int, cudaStream_t, bool);
@@ -260,7 +260,7 @@ int b200moe_gemm1(const b200moe_problem* p, const b200moe_workspace* ws, void* s
     return B200MOE_EINVAL;
   int sms;
   if ((rc = device_info(&sms))) return rc;
-  return launch_gemm1(p, ws, sms, static_cast<cudaStream_t>(stream));
+  return launch_gemm1(p, ws, sms, static_cast<cudaStream_t>(stream), false);
 }
 
 static int gemm2_stage(const b200moe_problem* p, const b200moe_workspace* ws, void* stream, bool half_out) {
@@ -270,7 +270,7 @@ static int gemm2_stage(const b200moe_problem* p, const b200moe_workspace* ws, vo
     return B200MOE_EINVAL;
   int sms;
   if ((rc = device_info(&sms))) return rc;
-  return launch_gemm2(p, ws, sms, static_cast<cudaStream_t>(stream), half_out);
+  return launch_gemm2(p, ws, sms, static_cast<cudaStream_t>(stream), half_out, false);
 }
 int b200moe_gemm2(const b200moe_problem* p, const b200moe_workspace* ws, void* stream) {
   return gemm2_stage(p, ws, stream, false);
@@ -401,11 +401,11 @@ int b200moe_forward(const b200moe_problem* p, const b200moe_workspace* ws, void*
     if ((rc = launch_gemm2_skinny(p, ws, sms, st, true))) return rc;
     return launch_reduce(p, ws, st, false);
   }
-  if ((rc = launch_gemm1(p, ws, sms, st))) return rc;
+  if ((rc = launch_gemm1(p, ws, sms, st, after_gather))) return rc;
   // Between the tile GEMM2 and the reduce of one call the per-expert rows live in the half form (eight float16 per
   // power-of-two scale byte): the two kernels are bound by writing and reading them.  (The stage entry points
   // b200moe_gemm2 / b200moe_reduce keep float32 rows.)
-  if ((rc = launch_gemm2(p, ws, sms, st, true))) return rc;
+  if ((rc = launch_gemm2(p, ws, sms, st, true, after_gather))) return rc;
   return launch_reduce(p, ws, st, true);
 }
 

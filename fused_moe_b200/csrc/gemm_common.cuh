@@ -21,8 +21,8 @@ struct GemmArgs {
   float* partial;            // token-minor kernels: partial sums of shared tiles, two slots per CTA
   int E_local;
   int R_max;
-  int early_weights;         // token-minor kernels inside b200moe_forward: weight stream starts before the dependency
-                             // wait, see gemm_skinny.cu
+  int early_weights;         // inside b200moe_forward: the weight stream starts before the dependency
+                             // wait, see the kernels
   int out_half;              // tile GEMM2: expert_out rows in the half form (half_rows.cuh) instead of float32
 };
 
