@@ -123,11 +123,13 @@ k_scatter(const int* __restrict__ topk_idx, const float* __restrict__ topk_w, lo
     for (int e = threadIdx.x; e <= E_local; e += blockDim.x) block_offsets[e] = s_row_base[e];
     if (threadIdx.x == 0) *total_blocks = tot_blocks;
   }
-  // pad rows: expert e is handled by CTA (e mod gridDim)
-  for (int e = blockIdx.x; e < E_local; e += gridDim.x) {
-    int begin = s_row_base[e] * BLOCK_M + (SCAN ? s_cnt[e] : __ldg(counts + e));
-    int end = s_row_base[e + 1] * BLOCK_M;
-    for (int r = begin + threadIdx.x; r < end; r += blockDim.x) {
+  // pad rows: a warp per expert.  (The grid has at least E_local warps.  With a grid for the chunks alone and a CTA per expert
+  // at a time, 40 tokens left one CTA to pad 256 experts one after the other: sort 19.4 us, now 4.6; 113 tokens / 128 experts
+  // 12.8 -> 4.7, 2048 / 256 10.2 -> 8.1, 80 / 32 5.9 -> 4.3, 16384 / 256 10.2 -> 10.6.)
+  for (int e = blockIdx.x * 4 + warp; e < E_local; e += gridDim.x * 4) {
+    const int begin = s_row_base[e] * BLOCK_M + (SCAN ? s_cnt[e] : __ldg(counts + e));
+    const int end = s_row_base[e + 1] * BLOCK_M;
+    for (int r = begin + lane; r < end; r += 32) {
       sorted_token_ids[r] = T;
       sorted_weights[r] = 0.f;
     }
@@ -464,7 +466,8 @@ int launch_sort(const b200moe_problem* p, const b200moe_workspace* ws, cudaStrea
     return B200MOE_OK;
   }
   const long long tstride = (!p->routing_logits && p->topk_row_stride) ? p->topk_row_stride : TOP_K;
-  int grid = (ws->n_chunks + 3) / 4;
+  const int work = ws->n_chunks > p->E_local ? ws->n_chunks : p->E_local;   // a warp per chunk and per expert
+  const int grid = (work + 3) / 4;
   if (ws->n_chunks <= SCATTER_SCAN_MAX_CHUNKS) {
     // small batch: the scatter CTAs do the scan themselves, one launch less
     B200MOE_CUDA_TRY(launch_pdl(k_scatter<true>, dim3(grid), dim3(128), 0, st, idx, w, tstride, ws->chunk_bits,
