@@ -269,8 +269,6 @@ def stage_times(K, inp, T, E_local, offset, reps=5, records=None):
     res = {}
     if records is None and _lib.uses_decode_path(T, E_local):
         names = ("route", "gemv1", "gemv2")          # decode path of b200moe_forward
-    elif records is None and T <= _lib.PROLOGUE_MAX_T:
-        names = ("prologue_small", "gemm1", "gemm2", "reduce")   # route + sort + gather are one launch here
     else:
         names = ("topk_bits" if records is not None else "route", "sort", "gather", "gemm1", "gemm2", "reduce")
     if records is None and T <= _lib.SKINNY_MAX_T:   # the GEMM kernels b200moe_forward uses at this batch size
@@ -622,8 +620,6 @@ def measure_workload(K, name, T_global, E1, skew, args, rank, world, device, pea
         launches_per_step = 17
     elif _l.uses_decode_path(T_loc, E_local):
         launches_per_step = 2          # route + GEMV1, GEMV2
-    elif T_loc <= _l.PROLOGUE_MAX_T:
-        launches_per_step = 4          # fused prologue, GEMM1, GEMM2, reduce
     elif T_loc <= 1024:
         launches_per_step = 6          # route, scatter (with the rank scan inside), gather, GEMM1, GEMM2, reduce
     else:

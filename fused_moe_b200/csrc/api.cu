@@ -380,32 +380,29 @@ int b200moe_forward(const b200moe_problem* p, const b200moe_workspace* ws, void*
     if ((rc = launch_route_gemv1(p, ws, sms, st))) return rc;
     return launch_gemv2(p, ws, sms, st);
   }
-  bool after_gather = false;   // GEMM1 directly follows k_gather (whose release tells it the sort is complete)
-  if (p->routing_logits && p->T <= B200MOE_PROLOGUE_MAX_T && !p->hidden_row_stride && !p->scale_token_stride && !p->scale_block_stride) {
-    // small batch: routing, ranking, layout, scatter and gather in one single-CTA kernel (same results)
-    if ((rc = launch_small_prologue(p, ws, st))) return rc;
+  // GEMM1 directly follows k_gather, whose release tells it that the sort is complete: its weight stream starts before the
+  // rows are there.  (Batches of up to 32 tokens used b200moe_prologue_small, one launch for these three, behind which GEMM1
+  // cannot start early: T = 20 / 32 experts 147.8 us per call against 144.7, skewed 82.4 / 79.0, T = 24 / 8 75.3 / 70.2,
+  // T = 32 / 256 821 / 808, T = 12 / 128 skewed 113.2 / 113.8.)
+  if (p->routing_logits) {
+    if ((rc = launch_route(p, ws, st))) return rc;
   } else {
-    after_gather = true;
-    if (p->routing_logits) {
-      if ((rc = launch_route(p, ws, st))) return rc;
-    } else {
-      if ((rc = launch_topk_bits(p, ws, st))) return rc;
-    }
-    if ((rc = launch_sort(p, ws, st))) return rc;
-    if ((rc = launch_gather(p, ws, sms, st))) return rc;
+    if ((rc = launch_topk_bits(p, ws, st))) return rc;
   }
+  if ((rc = launch_sort(p, ws, st))) return rc;
+  if ((rc = launch_gather(p, ws, sms, st))) return rc;
   // Few rows per expert (8 T / 256 per expert on average): token-minor tiles, bound by streaming the weights; else
   // 128-token tiles.  Both kernels are correct for every batch; the choice is about speed only.
   if (p->T <= B200MOE_SKINNY_MAX_T) {
-    if ((rc = launch_gemm1_skinny(p, ws, sms, st, after_gather))) return rc;
+    if ((rc = launch_gemm1_skinny(p, ws, sms, st, true))) return rc;
     if ((rc = launch_gemm2_skinny(p, ws, sms, st, true))) return rc;
     return launch_reduce(p, ws, st, false);
   }
-  if ((rc = launch_gemm1(p, ws, sms, st, after_gather))) return rc;
+  if ((rc = launch_gemm1(p, ws, sms, st, true))) return rc;
   // Between the tile GEMM2 and the reduce of one call the per-expert rows live in the half form (eight float16 per
   // power-of-two scale byte): the two kernels are bound by writing and reading them.  (The stage entry points
   // b200moe_gemm2 / b200moe_reduce keep float32 rows.)
-  if ((rc = launch_gemm2(p, ws, sms, st, true, after_gather))) return rc;
+  if ((rc = launch_gemm2(p, ws, sms, st, true, true))) return rc;
   return launch_reduce(p, ws, st, true);
 }
 

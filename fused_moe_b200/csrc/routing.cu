@@ -57,7 +57,8 @@ k_route(const float* __restrict__ logits, const uint16_t* __restrict__ bias, int
   }
 }
 
-// Small batches (T <= B200MOE_PROLOGUE_MAX_T): routing, ranking, padded layout, scatter and the activation gather in ONE launch instead of
+// The stage b200moe_prologue_small (T <= B200MOE_PROLOGUE_MAX_T), for hosts that pay more for a launch than b200moe_forward,
+// which runs the separate kernels: routing, ranking, padded layout, scatter and the activation gather in ONE launch instead of
 // four.  Same results, bit for bit, as k_route + k_rank_scan + k_scatter + k_gather.  Every CTA repeats the (cheap)
 // routing and layout of the whole batch in shared memory, so no CTA waits for another; CTA 0 alone writes the metadata
 // to global memory, and the row copies are dealt round-robin over all CTAs.  1024 threads: warp w routes token 32c + w

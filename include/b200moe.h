@@ -219,7 +219,8 @@ int b200moe_sort(const b200moe_problem* p, const b200moe_workspace* ws, void* st
 int b200moe_gather(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);
 /* b200moe_route + b200moe_sort + b200moe_gather in ONE launch for batches of at most B200MOE_PROLOGUE_MAX_T tokens with
  * dense inputs (all strides 0, routing_logits given); B200MOE_ETOOLARGE above that size, B200MOE_EINVAL for strided
- * inputs.  Leaves exactly the same workspace contents as the three stages.  b200moe_forward uses it for such batches.
+ * inputs.  Leaves exactly the same workspace contents as the three stages, which b200moe_forward launches one by one (its
+ * first GEMM can then start behind the gather).
  * Replaces, for such batches, the reference's routing + sort sequence (solution/python/pure_triton_impl.py:2207-2273). */
 int b200moe_prologue_small(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);
 /* Grouped FP8 GEMM1 with fp32 block-scale promotion every 128 K, SwiGLU, two-term e4m3 re-quantisation.
