@@ -481,8 +481,10 @@ class CudaExpertParallelMoE:
                 ready_event.record(torch.cuda.current_stream(device))
             return output
 
+        scale = K._host_scalar(routed_scaling_factor, float)   # once: reading a device scalar between two runs waits
+
         def layer(logits_dev, hs_dev, scale_dev, out_dev):
-            self.forward(logits_dev, routing_bias, hs_dev, scale_dev, routed_scaling_factor, out_dev)
+            self.forward(logits_dev, routing_bias, hs_dev, scale_dev, scale, out_dev)
 
         with torch.cuda.device(device):
             pipe = K.HostPipe.get(self.__dict__, "_host_pipe", device, T, (T + slices - 1) // slices)

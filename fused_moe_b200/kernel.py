@@ -13,6 +13,7 @@ from dataclasses import dataclass, field
 from typing import Dict, Optional, Tuple
 
 import torch
+from torch.utils.weak import WeakTensorKeyDictionary
 
 from . import _lib
 
@@ -59,18 +60,31 @@ class _DeviceState:
 
 
 _devices: Dict[int, _DeviceState] = {}
-_host_scalar_cache: Dict[tuple, object] = {}
+# Device scalars as last read outside a stream capture: tensor object (weakly) -> (its version then, value).  Only a call
+# under capture, which cannot read device memory, looks here.
+_read_scalars = WeakTensorKeyDictionary()
 
 
 def _host_scalar(x, cast):
-    """Python scalar from a scalar or a 0-d tensor; a device tensor is read back once per (address, dtype), as the
-    reference does (solution/python/pure_triton_impl.py:2012-2020)."""
-    if torch.is_tensor(x):
-        key = (x.data_ptr(), str(x.device), str(x.dtype), cast.__name__)
-        if key not in _host_scalar_cache:
-            _host_scalar_cache[key] = cast(x.item())
-        return _host_scalar_cache[key]
-    return cast(x)
+    """Python scalar from a number or a 0-d tensor.  A tensor is read on every call (a device tensor at the price of waiting
+    for the current stream): its value may have changed, and its address may be another tensor's by now.  The reference
+    reads a device tensor once per address (solution/python/pure_triton_impl.py:2012-2020).  Under stream capture a device
+    tensor cannot be read: the value that an earlier call read from this very tensor is taken if nothing has written to the
+    tensor since, and anything else is refused before the capture is touched."""
+    if not torch.is_tensor(x):
+        return cast(x)
+    if not x.is_cuda:
+        return cast(x.item())
+    if torch.cuda.is_current_stream_capturing():
+        version, value = _read_scalars.get(x, (None, None))
+        if version is None or version != x._version:
+            raise RuntimeError("a device scalar cannot be read during stream capture: pass a Python number or a CPU tensor, "
+                               "or make a call with the same tensor before the capture")
+        return cast(value)
+    value = x.item()
+    if not x.is_inference():   # inference tensors do not count their writes
+        _read_scalars[x] = (x._version, value)
+    return cast(value)
 
 
 def workspace_bytes(T: int, E_local: int) -> int:
@@ -229,10 +243,11 @@ def kernel(
 
     routing_logits [T,256] f32 · routing_bias [256] bf16 · hidden_states [T,7168] e4m3 · hidden_states_scale [56,T] f32 ·
     gemm1_weights [E,4096,7168] e4m3 · gemm1_weights_scale [E,32,56] f32 · gemm2_weights [E,7168,2048] e4m3 ·
-    gemm2_weights_scale [E,56,16] f32 · local_expert_offset, routed_scaling_factor: Python scalars or 0-d tensors ·
-    output: optional bf16 [T,7168] destination.  Returns the output tensor.  E (local experts) is taken from the weight
-    shape; the reference fixes it at 32.  Raises TypeError / ValueError on wrong dtypes or shapes and RuntimeError when
-    the CUDA library is missing, an input is not on a CUDA device, or a launch fails.
+    gemm2_weights_scale [E,56,16] f32 · local_expert_offset, routed_scaling_factor: Python scalars or 0-d tensors (one on
+    the device is read back on every call) · output: optional bf16 [T,7168] destination.  Returns the output tensor.  E
+    (local experts) is taken from the weight shape; the reference fixes it at 32.  Raises TypeError / ValueError on wrong
+    dtypes or shapes and RuntimeError when the CUDA library is missing, an input is not on a CUDA device, or a launch
+    fails.
     """
     if not torch.is_tensor(routing_logits) or routing_logits.dim() != 2:
         raise ValueError("routing_logits must be [T, 256]")
@@ -386,8 +401,10 @@ def kernel_host(routing_logits, routing_bias, hidden_states, hidden_states_scale
 
     def layer(logits_dev, hs_dev, scale_dev, out_dev):
         kernel(logits_dev, routing_bias, hs_dev, scale_dev, gemm1_weights, gemm1_weights_scale, gemm2_weights,
-               gemm2_weights_scale, local_expert_offset, routed_scaling_factor, out_dev)
+               gemm2_weights_scale, offset, scale, out_dev)
 
+    # once per call: reading a device scalar between two runs would wait for the first
+    offset, scale = _host_scalar(local_expert_offset, int), _host_scalar(routed_scaling_factor, float)
     with torch.cuda.device(device):
         pipe = HostPipe.get(_host_pipes, device.index, device, T, (T + slices - 1) // slices)
         return pipe.run(layer, logits, hs, hs_scale, output, slices, ready_event)
