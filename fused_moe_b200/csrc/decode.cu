@@ -406,7 +406,8 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
             m = fmaxf(m, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
 #pragma unroll
           for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-          const float k = m > 0.f ? 7.0f / m : 0.f;
+          m = fmaxf(m, 1e-36f);   // 7 / m stays finite (below 2.06e-38 it does not: inf, and NaN for zero elements)
+          const float k = 7.0f / m;
           uint4* dst = reinterpret_cast<uint4*>(dyn + static_cast<size_t>(r) * I * 2);
 #pragma unroll
           for (int i = 0; i < I / 16 / 32; ++i) {

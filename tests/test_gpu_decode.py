@@ -48,3 +48,40 @@ def test_decode_stages_equal_the_call(moe, T, E_local, skew):  # noqa: F811
             _lib.check(getattr(lib, "b200moe_" + stage)(C.byref(p), C.byref(ws.struct), stream), stage)
         torch.cuda.synchronize()
         assert torch.equal(out.view(T, 7168).to(torch.bfloat16), whole)
+
+
+def layer64(inp, E_local, offset=0):
+    """The layer in 64 bits on the same e4m3 values, scales and routing, [T, 7168]."""
+    from fused_moe_b200.kernel import route
+    idx, w = route(inp["routing_logits"], inp["routing_bias"], inp["routed_scaling_factor"])
+
+    def dequant(q, s):
+        r, c = q.shape
+        return (q.double().view(r // 128, 128, c // 128, 128) * s.double()[:, None, :, None]).view(r, c)
+
+    x = inp["hidden_states"].double().view(-1, 56, 128) * inp["hidden_states_scale"].t().double().unsqueeze(2)
+    x = x.view(-1, 7168)
+    out = torch.zeros_like(x)
+    for e in range(E_local):
+        token, k = (idx == offset + e).nonzero(as_tuple=True)
+        if token.numel():
+            up, gate = (x[token] @ dequant(inp["gemm1_weights"][e], inp["gemm1_weights_scale"][e]).t()).split(2048, dim=1)
+            y = (gate * torch.sigmoid(gate) * up) @ dequant(inp["gemm2_weights"][e], inp["gemm2_weights_scale"][e]).t()
+            out.index_add_(0, token, y * w[token, k].double().unsqueeze(1))
+    return out
+
+
+@pytest.mark.parametrize("T,E_local,skew,factor", [(8, 32, False, 3e-20), (8, 256, True, 3e-20), (2, 32, True, 1e-20)])
+def test_decode_keeps_small_rows(moe, T, E_local, skew, factor):  # noqa: F811
+    """Activation scales so small that the intermediate (quadratic in them) lies near the smallest normal float32, where the
+    reciprocal of a row's maximum overflows; W2 scales bring the result back into range."""
+    inp = dict(gpu_inputs(T, E_local, 44, 0, skew))
+    inp["hidden_states_scale"] = inp["hidden_states_scale"] * factor
+    inp["gemm2_weights_scale"] = inp["gemm2_weights_scale"] * 1e36
+    out = moe.kernel(**inp)
+    ref = layer64(inp, E_local)
+    assert torch.isfinite(out).all()
+    # bf16 rounding 1.7e-3 and the float32 intermediate's own step near 1e-39 (2^-149 / 1e-40: 1.4e-5)
+    assert (out.double() - ref).norm() <= 3e-3 * ref.norm()
+    inp["gemm2_weights_scale"] = gpu_inputs(T, E_local, 44, 0, skew)["gemm2_weights_scale"]
+    assert torch.isfinite(moe.kernel(**inp)).all()
