@@ -13,14 +13,18 @@
 //                   bytes a lane loads of a row are its A fragments, without a trip through shared memory.  Seven warps
 //                   take every seventh of the 56 K blocks of a task (a team reads 896 contiguous bytes per row at a time)
 //                   and add their sums through shared memory.
-//                   The instruction costs the same for one token and for eight, which is what it is for: packed half FMAs,
-//                   as in GEMV2, take 61 us instead of 26 for eight tokens on five hot experts (37 instead of 43 where
-//                   every expert has one token).  e4m3 mma.sync (m16n8k32) was slower: 40 us per call at T = 1 against 27.
-//   k_gemv2_reduce  GEMM2 and the weighted sum over experts on the CUDA cores.  A warp task is four output columns for the
-//                   whole batch: W2 rows in registers, the intermediate rows in shared memory as f16 scaled to |x| <= 7 by
-//                   their own maximum (11-bit rounding of each element, as the products'), packed half FMAs over 16 K
-//                   columns, fp32 from there on.  (The m16n8k16 form of it read 33 against 23 us at seven pairs.)
-//
+//                   The instruction costs the same for one token and for eight, which is what it is for: packed half FMAs
+//                   take 61 us instead of 26 for eight tokens on five hot experts (37 instead of 43 where every expert has
+//                   one token).  e4m3 mma.sync (m16n8k32) was slower: 40 us per call at T = 1 against 27.
+//   k_gemv2_reduce  GEMM2 and the weighted sum over experts with the same instruction.  A warp task is four output columns
+//                   for the whole batch: 8 KB of W2 per expert in registers, requested at once, the intermediate rows in
+//                   shared memory as f16 scaled per 128 columns (11-bit rounding of each element, the only one below 32
+//                   bits).  M = four columns x four quarters of K, so a warp needs no other warp's sums.
+//                   With packed half FMAs and one scale per row instead, the un-rounded sums were 4.9e-4 off 64 bits, now 1.7e-4
+//                   (one 128-column block 1e6 times larger than the others: 1.3e-2, now 1.7e-4).  us of the kernel, those / now:
+//                   one to eight pairs on experts of their own 14 / 14 .. 29 / 29, 22 pairs on four hot experts 35 / 30, 64 pairs
+//                   on 25 experts 100 / 96, on 46 experts 125 / 132 (~5.1 TB/s of W2).  Refilling the registers for the next
+//                   expert piece by piece took 140 there, independent chains of instructions changed nothing.
 // Measured: see the dispatch rule in api.cu.
 // Reference counterpart: the T = 1 path, solution/python/pure_triton_impl.py:2025-2123 (_kernel_t1) with
 // _t1_fused_gemm2_reduce_kernel (:1676-1750); oracle math solution/cuda/binding.py:157-182.
@@ -44,36 +48,28 @@ __device__ __forceinline__ uint4 ld_stream(const uint8_t* p) {
                : "l"(p));
   return v;
 }
-// 16 e4m3 values -> f16, exactly.
-struct Half2x8 {
-  __half2 v[8];
-};
-__device__ __forceinline__ Half2x8 cvt16_h2(const uint4& q) {
-  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-  Half2x8 r;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    __half2_raw lo = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w[i] & 0xffffu), __NV_E4M3);
-    __half2_raw hi = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w[i] >> 16), __NV_E4M3);
-    r.v[2 * i] = *reinterpret_cast<__half2*>(&lo);
-    r.v[2 * i + 1] = *reinterpret_cast<__half2*>(&hi);
-  }
-  return r;
-}
 __device__ __forceinline__ uint32_t half2_bits(const __half2& h) { return *reinterpret_cast<const uint32_t*>(&h); }
+// Four e4m3 values -> f16, exactly.
+__device__ __forceinline__ uint2 cvt4_h2(uint32_t w) {
+  const __half2_raw a = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w & 0xffffu), __NV_E4M3);
+  const __half2_raw b = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w >> 16), __NV_E4M3);
+  return make_uint2(half2_bits(__half2(a)), half2_bits(__half2(b)));
+}
+// c += 16 K columns: a0 / a1 = the lane's four of M rows g and g + 8, b0 b1 = the same four of N column g.
+__device__ __forceinline__ void mma_k16(float (&c)[4], const uint2& a0, const uint2& a1, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0.x), "r"(a1.x), "r"(a0.y), "r"(a1.y), "r"(b0), "r"(b1));
+}
 // c += 64 K columns of 16 weight rows x 8 tokens.  lo / hi: the lane's 16 weights of M rows g and g + 8; b: the same 16 K
 // columns of token g (f16).  Four MMAs, each taking four of the lane's columns.
 __device__ __forceinline__ void mma_k64(float (&c)[4], const uint4& lo, const uint4& hi, const uint8_t* b) {
-  const Half2x8 x = cvt16_h2(lo), y = cvt16_h2(hi);
   const uint4 b0 = reinterpret_cast<const uint4*>(b)[0], b1 = reinterpret_cast<const uint4*>(b)[1];
-  const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(half2_bits(x.v[2 * j])), "r"(half2_bits(y.v[2 * j])), "r"(half2_bits(x.v[2 * j + 1])),
-          "r"(half2_bits(y.v[2 * j + 1])), "r"(bw[2 * j]), "r"(bw[2 * j + 1]));
+  mma_k16(c, cvt4_h2(lo.x), cvt4_h2(hi.x), b0.x, b0.y);
+  mma_k16(c, cvt4_h2(lo.y), cvt4_h2(hi.y), b0.z, b0.w);
+  mma_k16(c, cvt4_h2(lo.z), cvt4_h2(hi.z), b1.x, b1.y);
+  mma_k16(c, cvt4_h2(lo.w), cvt4_h2(hi.w), b1.z, b1.w);
 }
 // Ask for bytes [p, p + bytes) to be brought into L2 (16-byte aligned, a multiple of 16; no completion to wait for).
 __device__ __forceinline__ void l2_prefetch_bulk(const void* p, uint32_t bytes) {
@@ -129,7 +125,7 @@ __device__ __forceinline__ void build_lists(ExpertLists& L, int E_local) {
 // ---------------------------------------------------------------------------------------------------------
 constexpr int G1_TEAM_WARPS = 7;                          // 56 K blocks, eight per warp
 constexpr int G1_TEAMS = 2;
-constexpr int G1_THREADS = G1_TEAMS * G1_TEAM_WARPS * 32; // 448: 144 registers per thread
+constexpr int G1_THREADS = G1_TEAMS * G1_TEAM_WARPS * 32; // 448: four warps on a quarter of the SM, 128 registers per thread
 constexpr int G1_COLS = 8;
 constexpr int G1_ROW = 2 * H + 16;        // pitch of an activation row: tokens 16 bytes apart modulo 128, B loads without conflicts
 constexpr int G1_SCALES = H_BLOCKS + 1;
@@ -161,10 +157,11 @@ k_gemv1_swiglu(const float* __restrict__ logits, const uint16_t* __restrict__ bi
   pdl_launch_dependents();
   for (int c = threadIdx.x; c < T * (H / 16); c += G1_THREADS) {
     const int t = c / (H / 16), u = c - t * (H / 16);
-    const Half2x8 h = cvt16_h2(__ldg(reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(t) * H) + u));
+    const uint4 h = __ldg(reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(t) * H) + u);
+    const uint2 h0 = cvt4_h2(h.x), h1 = cvt4_h2(h.y), h2 = cvt4_h2(h.z), h3 = cvt4_h2(h.w);
     uint4* dst = reinterpret_cast<uint4*>(rows + t * G1_ROW + u * 32);
-    dst[0] = *reinterpret_cast<const uint4*>(&h.v[0]);
-    dst[1] = *reinterpret_cast<const uint4*>(&h.v[4]);
+    dst[0] = make_uint4(h0.x, h0.y, h1.x, h1.y);
+    dst[1] = make_uint4(h2.x, h2.y, h3.x, h3.y);
   }
   for (int c = threadIdx.x; c < T * H_BLOCKS; c += G1_THREADS) {
     const int kb = c / T, t = c - kb * T;
@@ -285,72 +282,91 @@ k_gemv1_swiglu(const float* __restrict__ logits, const uint16_t* __restrict__ bi
 // ---------------------------------------------------------------------------------------------------------
 // GEMM2 + weighted sum over experts
 // ---------------------------------------------------------------------------------------------------------
-// 16 K columns of one weight row (already f16) against one token's activations.
-__device__ __forceinline__ float dot16_h2(const Half2x8& a, const Half2x8& w) {
-  __half2 acc = __hmul2(a.v[0], w.v[0]);
-#pragma unroll
-  for (int i = 1; i < 8; ++i) acc = __hfma2(a.v[i], w.v[i], acc);
-  const float2 f = __half22float2(acc);
-  return f.x + f.y;
-}
-
 // Hides from the compiler that `w` is the same in every round of a loop.  Without it the f16 form of all weights a thread
 // holds is computed once before the loop over an expert's tokens (usually one): twice the registers, spilled.
 __device__ __forceinline__ void keep_packed(uint4& w) {
   asm volatile("" : "+r"(w.x), "+r"(w.y), "+r"(w.z), "+r"(w.w));
 }
 
-// The staged activation of token t (GEMV1): chunk c = 16 columns, two 16-byte units in swizzled order.
-__device__ __forceinline__ Half2x8 staged16(const uint4* row, int c) {
-  const int sw = (c >> 2) & 1;
-  Half2x8 a;
-  *reinterpret_cast<uint4*>(&a.v[0]) = row[2 * c + sw];
-  *reinterpret_cast<uint4*>(&a.v[4]) = row[2 * c + (sw ^ 1)];
-  return a;
-}
-
 constexpr int G2_WARPS = 16;
 constexpr int G2_THREADS = G2_WARPS * 32;
 constexpr int GEMV2_BATCH = 24;   // intermediate rows staged at a time (4 KB each)
 constexpr int GEMV2_COLS = 4;     // output columns per warp task
+constexpr int GEMV2_STEPS = I / 256;   // a lane's 16-byte pieces of a weight row
+constexpr int G2_ROW = 2 * I + 16;   // pitch of a staged row: the rows of a token pair 16 bytes apart modulo 128
 
-// M intermediate rows (pairs q ..) of one expert against four rows of W2, converted to f16 once for all M; lane 8 c + t
-// adds column c of token t.
-template <int M>
-__device__ __forceinline__ void gemv2_rows(int q, int p0, int lane, const uint8_t* staged,
-                                           uint4 (&w)[GEMV2_COLS][I / 16 / 32], const float (&f)[I / 16 / 32],
-                                           const uint8_t* token, const float* s_back, float& tot) {
-  float acc[M][GEMV2_COLS];
+struct Gemv2Shared {
+  uint8_t row[GEMV2_BATCH + 1][G2_ROW];          // f16, scaled to |x| <= 256 per 128 columns
+  float scale[I_BLOCKS][GEMV2_BATCH + 1];        // what undoes it, times the routing weight
+  ExpertLists L;
+};
+
+// P pairs of tokens (list entries r .., rows r - p0 .. of the staged batch; `n` of the 2 P are real) of one expert against
+// four rows of W2.  M rows 4 c + j and 8 + 4 c + j: quarter j of the K columns of columns c and 2 + c; N column 2 j + t: the
+// same quarter of token t of the pair.  Quarter 2 a + b is half b (64 columns) of each of the 128-column blocks 8 a .. 8 a + 7:
+// the eight lanes of a (column, a) read whole lines.  Only equal quarters belong together, so lane 16 c + 5 j holds four
+// sums and the others nothing of use; that costs the tensor core three quarters of its work, of which it has plenty, and
+// keeps each warp's weights, sums and columns to itself.  Lane 8 c + t adds column c of token t to `tot`.
+template <int P>
+__device__ __forceinline__ void gemv2_rows(const Gemv2Shared& S, int r, int p0, int n, int lane,
+                                           uint4 (&w)[GEMV2_STEPS][2], float w_scale, float& tot) {
+  const int g = lane >> 2, q = lane & 3;
+  // Slots past the last token take whatever the next row holds (the arrays have a row more for that): an N column's sums come
+  // from its own values alone, and those of such a slot are not used.
+  const uint8_t* b = S.row[r - p0 + (g & 1)] + (g >> 2) * (GEMV2_STEPS * 256) + (g >> 1 & 1) * 128 + q * 32;
+  const float* x = &S.scale[(q >> 1) * GEMV2_STEPS][r - p0];
+  float acc[P][4];
 #pragma unroll
-  for (int r = 0; r < M; ++r)
+  for (int p = 0; p < P; ++p)
 #pragma unroll
-    for (int j = 0; j < GEMV2_COLS; ++j) acc[r][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[p][j] = 0.f;
 #pragma unroll
-  for (int i = 0; i < I / 16 / 32; ++i) {
-    Half2x8 a[M];
+  for (int i = 0; i < GEMV2_STEPS; ++i) {
+    keep_packed(w[i][0]);
+    keep_packed(w[i][1]);
+    const uint32_t lo[4] = {w[i][0].x, w[i][0].y, w[i][0].z, w[i][0].w}, hi[4] = {w[i][1].x, w[i][1].y, w[i][1].z, w[i][1].w};
+    float c[P][4];
 #pragma unroll
-    for (int r = 0; r < M; ++r)
-      a[r] = staged16(reinterpret_cast<const uint4*>(staged + static_cast<size_t>(q - p0 + r) * I * 2), i * 32 + lane);
+    for (int p = 0; p < P; ++p)
 #pragma unroll
-    for (int j = 0; j < GEMV2_COLS; ++j) {
-      keep_packed(w[j][i]);
-      const Half2x8 h = cvt16_h2(w[j][i]);
+      for (int j = 0; j < 4; ++j) c[p][j] = 0.f;
 #pragma unroll
-      for (int r = 0; r < M; ++r) acc[r][j] = fmaf(dot16_h2(a[r], h), f[i], acc[r][j]);
+    for (int h = 0; h < 2; ++h) {
+      uint4 bv[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) bv[p] = *reinterpret_cast<const uint4*>(b + p * (2 * G2_ROW) + i * 256 + h * 16);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint2 a0 = cvt4_h2(lo[2 * h + k]), a1 = cvt4_h2(hi[2 * h + k]);
+#pragma unroll
+        for (int p = 0; p < P; ++p) mma_k16(c[p], a0, a1, k ? bv[p].z : bv[p].x, k ? bv[p].w : bv[p].y);
+      }
+    }
+    const float f = __shfl_sync(0xffffffffu, w_scale, (g >> 1 & 1) * GEMV2_STEPS + i);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const float f0 = x[i * (GEMV2_BATCH + 1) + 2 * p] * f, f1 = x[i * (GEMV2_BATCH + 1) + 2 * p + 1] * f;
+      acc[p][0] = fmaf(c[p][0], f0, acc[p][0]);
+      acc[p][1] = fmaf(c[p][1], f1, acc[p][1]);
+      acc[p][2] = fmaf(c[p][2], f0, acc[p][2]);
+      acc[p][3] = fmaf(c[p][3], f1, acc[p][3]);
     }
   }
 #pragma unroll
-  for (int r = 0; r < M; ++r) {
-    // four sums over 32 lanes; lanes 8 c .. 8 c + 7 end up with the sum of column c
-    const bool hi = (lane & 16) != 0, mid = (lane & 8) != 0;
-    float x0 = hi ? acc[r][2] : acc[r][0], x1 = hi ? acc[r][3] : acc[r][1];
-    x0 += __shfl_xor_sync(0xffffffffu, hi ? acc[r][0] : acc[r][2], 16);
-    x1 += __shfl_xor_sync(0xffffffffu, hi ? acc[r][1] : acc[r][3], 16);
-    float y = mid ? x1 : x0;
-    y += __shfl_xor_sync(0xffffffffu, mid ? x0 : x1, 8);
+  for (int p = 0; p < P; ++p) {
+    // add the four quarters (lanes 16 c + 5 j); afterwards lane 16 c + 5 (k + 2 t) holds column c + 2 k of token t
+    const bool hi = (lane & 1) != 0, odd = (lane & 2) != 0;
+    float y0 = hi ? acc[p][2] : acc[p][0], y1 = hi ? acc[p][3] : acc[p][1];
+    y0 += __shfl_xor_sync(0xffffffffu, hi ? acc[p][0] : acc[p][2], 5);
+    y1 += __shfl_xor_sync(0xffffffffu, hi ? acc[p][1] : acc[p][3], 5);
+    float z = odd ? y1 : y0;
+    z += __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 10);
+    const int src = (lane & 8) * 2 + (lane >> 4) * 5;
 #pragma unroll
-    for (int d = 4; d > 0; d >>= 1) y += __shfl_xor_sync(0xffffffffu, y, d);
-    if ((lane & 7) == token[q + r]) tot = fmaf(s_back[q - p0 + r], y, tot);
+    for (int t = 0; t < 2; ++t) {
+      const float v = __shfl_sync(0xffffffffu, z, src + 10 * t);
+      if (2 * p + t < n && (lane & 7) == S.L.token[r + 2 * p + t]) tot += v;
+    }
   }
 }
 
@@ -359,9 +375,9 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
 k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx, const float* __restrict__ topk_w,
                int T, int local_offset, int E_local, const uint8_t* __restrict__ w2, const float* __restrict__ w2_scale,
                uint16_t* __restrict__ out, float* __restrict__ out_f32) {
-  extern __shared__ __align__(16) uint8_t dyn[];         // GEMV2_BATCH rows of 2048 f16
-  __shared__ float s_back[GEMV2_BATCH];                  // weight * row maximum / 7
-  __shared__ ExpertLists L;
+  extern __shared__ __align__(16) uint8_t dyn[];
+  Gemv2Shared& S = *reinterpret_cast<Gemv2Shared*>(dyn);
+  ExpertLists& L = S.L;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int G = gridDim.x;
   if (threadIdx.x < E_GLOBAL) L.mask[threadIdx.x] = 0;
@@ -391,42 +407,36 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
       const int p1 = p0 + GEMV2_BATCH < n_pairs ? p0 + GEMV2_BATCH : n_pairs;
       if (staged != p0) {
         if (staged >= 0) __syncthreads();   // everybody has finished with the rows that are replaced
-        // one warp per row: f16 scaled to |x| <= 7 by the row's own maximum (11-bit rounding of each element)
+        // a warp per 512 columns of a row: f16 scaled to |x| <= 256 by the largest magnitude of each 128 (eight lanes' share)
 #pragma unroll 1
-        for (int r = warp; r < p1 - p0; r += G2_WARPS) {
-          const float4* x = reinterpret_cast<const float4*>(inter + static_cast<size_t>(p0 + r) * I);
-          float4 v[I / 4 / 32];
-          float m = 0.f;
+        for (int h = warp; h < 4 * (p1 - p0); h += G2_WARPS) {
+          const int r = h >> 2, c = (h & 3) * 32 + lane;   // this lane's 16 columns
+          const float4* x = reinterpret_cast<const float4*>(inter + static_cast<size_t>(p0 + r) * I) + c * 4;
+          float4 v[4];
 #pragma unroll
-          for (int i = 0; i < I / 16 / 32; ++i)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v[4 * i + q] = __ldg(x + (i * 32 + lane) * 4 + q);
-#pragma unroll
-          for (int i = 0; i < I / 4 / 32; ++i)
-            m = fmaxf(m, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
-#pragma unroll
-          for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-          m = fmaxf(m, 1e-36f);   // 7 / m stays finite (below 2.06e-38 it does not: inf, and NaN for zero elements)
-          const float k = 7.0f / m;
-          uint4* dst = reinterpret_cast<uint4*>(dyn + static_cast<size_t>(r) * I * 2);
-#pragma unroll
-          for (int i = 0; i < I / 16 / 32; ++i) {
-            Half2x8 a;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              a.v[2 * q] = __floats2half2_rn(v[4 * i + q].x * k, v[4 * i + q].y * k);
-              a.v[2 * q + 1] = __floats2half2_rn(v[4 * i + q].z * k, v[4 * i + q].w * k);
-            }
-            const int c = i * 32 + lane, sw = (c >> 2) & 1;
-            dst[2 * c + sw] = *reinterpret_cast<const uint4*>(&a.v[0]);
-            dst[2 * c + (sw ^ 1)] = *reinterpret_cast<const uint4*>(&a.v[4]);
-          }
-          // the slot k in which the pair's token holds the pair's expert
+          for (int q = 0; q < 4; ++q) v[q] = __ldg(x + q);
+          // the routing weight: the slot in which the pair's token holds the pair's expert
           int u_r = 0;
           while (L.first[u_r + 1] <= p0 + r) ++u_r;
-          const int t = L.token[p0 + r];
-          const bool hit = lane < TOP_K && __ldg(topk_idx + t * TOP_K + lane) == L.e[u_r] + local_offset;
-          if (hit) s_back[r] = __ldg(topk_w + t * TOP_K + lane) * m * (1.0f / 7.0f);
+          const int at = L.token[p0 + r] * TOP_K + (lane & (TOP_K - 1));
+          const float wk = __ldg(topk_w + at);
+          const uint32_t hit = __ballot_sync(0xffffffffu, __ldg(topk_idx + at) == L.e[u_r] + local_offset);
+          const float weight = __shfl_sync(0xffffffffu, wk, __ffs(hit) - 1);
+          float m = 1e-36f;   // 256 / m stays finite
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v[q].x), fabsf(v[q].y)), fmaxf(fabsf(v[q].z), fabsf(v[q].w))));
+#pragma unroll
+          for (int d = 4; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+          const float k = 256.0f / m;
+          uint4* dst = reinterpret_cast<uint4*>(S.row[r] + c * 32);
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const float4 &a = v[2 * q], &b = v[2 * q + 1];
+            dst[q] = make_uint4(half2_bits(__floats2half2_rn(a.x * k, a.y * k)), half2_bits(__floats2half2_rn(a.z * k, a.w * k)),
+                                half2_bits(__floats2half2_rn(b.x * k, b.y * k)), half2_bits(__floats2half2_rn(b.z * k, b.w * k)));
+          }
+          if ((lane & 7) == 0) S.scale[c >> 3][r] = weight * (m * (1.0f / 256.0f));
         }
         staged = p0;
         __syncthreads();
@@ -434,22 +444,21 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
       if (g >= g_end) continue;
       while (u < n_lists && L.first[u] < p1) {
         const int e = L.e[u];
-        const uint4* w_row = reinterpret_cast<const uint4*>(w2 + (static_cast<size_t>(e) * H + n0) * I) + lane;
-        const float* sc = w2_scale + (static_cast<size_t>(e) * H_BLOCKS + (n0 >> 7)) * I_BLOCKS + (lane >> 3);
-        uint4 w[GEMV2_COLS][I / 16 / 32];
-        float f[I / 16 / 32];
+        // this lane's 64-column halves of the blocks 8 a + i of columns n0 + c and n0 + 2 + c (lane = 16 c + 8 a + 4 b + q)
+        const uint8_t* w_row = w2 + (static_cast<size_t>(e) * H + n0 + (lane >> 4)) * I + (lane >> 3 & 1) * (GEMV2_STEPS * 128) + (lane & 7) * 16;
+        uint4 w[GEMV2_STEPS][2];
 #pragma unroll
-        for (int j = 0; j < GEMV2_COLS; ++j)
+        for (int i = 0; i < GEMV2_STEPS; ++i)
 #pragma unroll
-          for (int i = 0; i < I / 16 / 32; ++i) w[j][i] = ld_stream(reinterpret_cast<const uint8_t*>(w_row + j * (I / 16) + i * 32));
-#pragma unroll
-        for (int i = 0; i < I / 16 / 32; ++i) f[i] = __ldg(sc + 4 * i);
+          for (int j = 0; j < 2; ++j) w[i][j] = ld_stream(w_row + j * (2 * I) + i * 128);
+        // lanes 0..15: the scales of the 16 K blocks
+        const float w_scale = __ldg(w2_scale + (static_cast<size_t>(e) * H_BLOCKS + (n0 >> 7)) * I_BLOCKS + (lane & (I_BLOCKS - 1)));
         const int first = L.first[u], last = L.first[u + 1];
-        const int q1 = last < p1 ? last : p1;
-        int q = first > p0 ? first : p0;
+        const int r1 = last < p1 ? last : p1;
+        int r = first > p0 ? first : p0;
 #pragma unroll 1
-        for (; q + 1 < q1; q += 2) gemv2_rows<2>(q, p0, lane, dyn, w, f, L.token, s_back, tot);
-        if (q < q1) gemv2_rows<1>(q, p0, lane, dyn, w, f, L.token, s_back, tot);
+        for (; r + 2 < r1; r += 4) gemv2_rows<2>(S, r, p0, min(r1 - r, 4), lane, w, w_scale, tot);
+        if (r < r1) gemv2_rows<1>(S, r, p0, r1 - r, lane, w, w_scale, tot);
         if (last > p1) break;   // the rest of this expert's tokens are in the next batch of rows
         ++u;
       }
@@ -517,7 +526,7 @@ int launch_gemv2(const b200moe_problem* p, const b200moe_workspace* ws, int num_
   if (p->T == 0) return B200MOE_OK;
   static bool attr_set[64] = {};
   int dev = 0;
-  constexpr int SMEM = GEMV2_BATCH * I * 2;
+  constexpr int SMEM = sizeof(Gemv2Shared);
   B200MOE_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 64 && !attr_set[dev]) {
     B200MOE_CUDA_TRY(cudaFuncSetAttribute(k_gemv2_reduce, cudaFuncAttributeMaxDynamicSharedMemorySize,

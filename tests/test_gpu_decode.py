@@ -85,3 +85,33 @@ def test_decode_keeps_small_rows(moe, T, E_local, skew, factor):  # noqa: F811
     assert (out.double() - ref).norm() <= 3e-3 * ref.norm()
     inp["gemm2_weights_scale"] = gpu_inputs(T, E_local, 44, 0, skew)["gemm2_weights_scale"]
     assert torch.isfinite(moe.kernel(**inp)).all()
+
+
+@pytest.mark.parametrize("T,E_local,skew", [(1, 128, False), (7, 32, False), (8, 32, True), (8, 256, True), (4, 1, False)])
+@pytest.mark.parametrize("wide", [1.0, 1e6])
+def test_decode_sums_keep_32_bits(moe, T, E_local, skew, wide):  # noqa: F811
+    """The un-rounded sums against 64 bits.  The one rounding below 32 bits is the intermediate's to float16, whose relative
+    error has a root mean square of 2.1e-4 over a binade and no weight in which to add up: so much is left of it in the
+    2-norm of the result.  Also where one 128-column block of the intermediate is `wide` times larger than the others and
+    its W2 scale as much smaller."""
+    from fused_moe_b200 import _lib
+    from fused_moe_b200.kernel import _problem, route
+    inp = dict(gpu_inputs(T, E_local, 43, 0, skew))
+    if E_local == 1:   # every token on the one expert
+        inp["routing_logits"] = inp["routing_logits"].clone()
+        inp["routing_logits"][:, 0] += 20.0
+        assert (route(inp["routing_logits"], inp["routing_bias"], 2.5)[0] == 0).any(dim=1).all()
+    for name, at, f in (("gemm1_weights_scale", (slice(None), 5), wide), ("gemm2_weights_scale", (slice(None), slice(None), 5), 1 / wide)):
+        inp[name] = inp[name].clone()
+        inp[name][at] *= f
+    moe.kernel(**inp)
+    ws = moe.last_workspace()
+    out = torch.full((T, 7168), 3.0, device="cuda")
+    p = _problem(T, E_local, 0, float(inp["routed_scaling_factor"]), inp["routing_logits"], inp["routing_bias"],
+                 inp["hidden_states"], inp["hidden_states_scale"], inp["gemm1_weights"], inp["gemm1_weights_scale"],
+                 inp["gemm2_weights"], inp["gemm2_weights_scale"], out)
+    _lib.check(_lib.load().b200moe_forward(C.byref(p), C.byref(ws.struct), torch.cuda.current_stream().cuda_stream), "forward")
+    ref = layer64(inp, E_local)
+    err = ((out.double() - ref).norm() / ref.norm()).item()
+    print(f"T={T} E={E_local} skew={skew} wide={wide:g}: {err:.3g}")
+    assert err <= 2.6e-4
