@@ -15,13 +15,13 @@ OK, EINVAL, EWORKSPACE, ECUDA, EDEVICE, EUNSUPPORTED, ETOOLARGE = 0, -1, -2, -3,
 SORT_STATIC_MAX_ENTRIES = 32768
 EP_RECORD_BYTES = 7456
 DECODE_MAX_T = 8
-DECODE_MAX_WORK = 2048
+DECODE_MAX_WORK = 2048   # limits nothing: eight tokens x 256 experts
 
 
 def uses_decode_path(T: int, E_local: int) -> bool:
-    """Whether b200moe_forward takes the matrix-vector stages for a routed call with dense inputs (at most eight tokens:
-    an expert's tokens then fill one N = 8 tile of the instruction that the stages use)."""
-    return T <= DECODE_MAX_T and T * E_local <= DECODE_MAX_WORK
+    """Whether b200moe_forward takes the matrix-vector stages for a routed call with dense inputs: at most eight tokens
+    (an expert's tokens then fill one N = 8 tile of the instruction that the stages use), with any number of experts."""
+    return T <= DECODE_MAX_T
 
 PROLOGUE_MAX_T = 32
 SKINNY_MAX_T = 112

@@ -370,13 +370,13 @@ int b200moe_forward(const b200moe_problem* p, const b200moe_workspace* ws, void*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // Decode, at most eight tokens: every expert's tokens fit one N = 8 instruction and the whole batch's activations fit
   // shared memory, so nothing has to be sorted or gathered and the weights go from HBM to the tensor core through
-  // registers.  Measured at the limit and below it (us per call, this path / the sorted path; E = local experts, skewed =
-  // hot experts that several tokens share): T = 8, E = 32 69 / 99, skewed 61 / 73; T = 8, E = 256 342 / 389, skewed
-  // 221 / 236; T = 8, E = 128 skewed 102 / 103; T = 1, E = 256 67 / 103; T = 6, E = 8 skewed 25 / 49.  Past eight tokens the
-  // f16 activations take the shared memory that the weight loads in flight need as L1 (T = 14, E = 32: 212 / 138).
-  if (p->routing_logits && p->T <= B200MOE_DECODE_MAX_T && p->T * p->E_local <= B200MOE_DECODE_MAX_WORK &&
-      p->out_seg_count == 0 && p->partial_format == B200MOE_PARTIAL_F32 && !p->hidden_row_stride &&
-      !p->scale_token_stride && !p->scale_block_stride) {
+  // registers, whatever the number of local experts.  Measured at the limit and below it (us per call among others, means over
+  // twelve batches, this path / the sorted path; E = local experts, skewed = hot experts that several tokens share): T = 8,
+  // E = 32 58 / 85, skewed 50 / 69; T = 8, E = 256 359 / 403, skewed 190 / 218; T = 8, E = 128 skewed 101 / 122; T = 1, E = 256
+  // 73 / 108, E = 32 23 / 55; T = 6, E = 8 skewed 22 / 51; T = 8, E = 1 18 / 49.  Past eight tokens the f16 activations take the
+  // shared memory that the weight loads in flight need as L1 (T = 14, E = 32: 212 / 138).
+  if (p->routing_logits && p->T <= B200MOE_DECODE_MAX_T && p->out_seg_count == 0 &&
+      p->partial_format == B200MOE_PARTIAL_F32 && !p->hidden_row_stride && !p->scale_token_stride && !p->scale_block_stride) {
     if ((rc = launch_route_gemv1(p, ws, sms, st))) return rc;
     return launch_gemv2(p, ws, sms, st);
   }

@@ -356,7 +356,8 @@ def kernel_host(routing_logits, routing_bias, hidden_states, hidden_states_scale
     ``hidden_states_scale`` and ``output`` are pinned host tensors (``output=None`` allocates one), the bias and the
     expert weights are device tensors as in ``kernel``.  The tokens are cut into ``slices`` equal runs and pipelined
     over three streams, so the host-to-device copy of run i + 1 and the device-to-host copy of run i - 1 overlap the
-    layer on run i; rows are independent, so the result equals one ``kernel`` call on all tokens bit for bit.
+    layer on run i; rows are independent, so the result equals one ``kernel`` call on all tokens: bit for bit
+    where every run has more than 112 tokens (the same kernels), within the layer's tolerance otherwise.
     Returns ``output`` after queueing everything.
 
     Without ``ready_event`` the caller's current stream waits for the last copy, so synchronising that stream (or the

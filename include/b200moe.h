@@ -41,9 +41,10 @@ extern "C" {
 #define B200MOE_SKINNY_MAX_T 112   /* b200moe_forward uses the token-minor GEMM kernels up to this batch size */
 #endif
 #define B200MOE_PROLOGUE_MAX_T 32  /* largest batch of b200moe_prologue_small */
-#define B200MOE_DECODE_MAX_T 8 /* the matrix-vector (decode) stages take at most this many tokens; b200moe_forward
-                                  uses them while T * E_local <= B200MOE_DECODE_MAX_WORK */
-#define B200MOE_DECODE_MAX_WORK 2048 /* every number of local experts: eight tokens x 256 */
+#define B200MOE_DECODE_MAX_T 8 /* the matrix-vector (decode) stages take at most this many tokens, and b200moe_forward uses
+                                  them up to here */
+#define B200MOE_DECODE_MAX_WORK 2048 /* largest T * E_local of the decode stages.  It limits nothing (eight tokens x 256
+                                        experts); kept for callers that compare with it */
 
 enum {
   B200MOE_OK = 0,
@@ -183,10 +184,12 @@ int b200moe_workspace_carve(void* base, size_t bytes, int32_t T, int32_t E_local
 int b200moe_workspace_init(const b200moe_workspace* ws /* host */, void* stream);
 
 /* Whole layer: route -> rank -> scatter -> gather -> GEMM1+SwiGLU -> GEMM2 -> weighted reduce, all on `stream`,
- * no host synchronisation.  With routing_logits given, T <= B200MOE_DECODE_MAX_T and T * E_local <=
- * B200MOE_DECODE_MAX_WORK it runs (route + GEMV1 + SwiGLU) -> (GEMV2 + reduce) instead, two launches with the results of
- * b200moe_route, b200moe_gemv1, b200moe_gemv2 below: no sort, no gather, fp32 intermediate.  Replaces solution/python/pure_triton_impl.py:2125-2403 (kernel), :2025-2123 (_kernel_t1),
- * solution/python/triton_impl.py:346-566 and solution/python/triton_impl_t901.py:40-185. */
+ * no host synchronisation.  With routing_logits given, T <= B200MOE_DECODE_MAX_T, dense inputs,
+ * no output segments and float32 or bf16 rows out it runs (route + GEMV1 + SwiGLU) -> (GEMV2 + reduce) instead, two launches
+ * with the results of b200moe_route, b200moe_gemv1, b200moe_gemv2 below: no sort, no gather, fp32 intermediate; counts,
+ * block_offsets, total_blocks, scatter_map and the sorted arrays are then left as they were.  Replaces
+ * solution/python/pure_triton_impl.py:2125-2403 (kernel), :2025-2123 (_kernel_t1), solution/python/triton_impl.py:346-566
+ * and solution/python/triton_impl_t901.py:40-185. */
 int b200moe_forward(const b200moe_problem* p /* host */, const b200moe_workspace* ws /* host */, void* stream);
 
 /* Upstream of the layer: bf16 activations [T, 7168] -> e4m3 [T, 7168] and float32 scales [56, T], one scale per token
@@ -219,8 +222,8 @@ int b200moe_sort(const b200moe_problem* p, const b200moe_workspace* ws, void* st
 int b200moe_gather(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);
 /* b200moe_route + b200moe_sort + b200moe_gather in ONE launch for batches of at most B200MOE_PROLOGUE_MAX_T tokens with
  * dense inputs (all strides 0, routing_logits given); B200MOE_ETOOLARGE above that size, B200MOE_EINVAL for strided
- * inputs.  Leaves exactly the same workspace contents as the three stages, which b200moe_forward launches one by one (its
- * first GEMM can then start behind the gather).
+ * inputs.  Leaves what the three stages leave (and chunk_base, which b200moe_sort writes above 1024 tokens only);
+ * b200moe_forward launches the three one by one (its first GEMM can then start behind the gather).
  * Replaces, for such batches, the reference's routing + sort sequence (solution/python/pure_triton_impl.py:2207-2273). */
 int b200moe_prologue_small(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);
 /* Grouped FP8 GEMM1 with fp32 block-scale promotion every 128 K, SwiGLU, two-term e4m3 re-quantisation.
@@ -239,7 +242,8 @@ int b200moe_gemm2(const b200moe_problem* p, const b200moe_workspace* ws, void* s
 int b200moe_gemm1_skinny(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);
 int b200moe_gemm2_skinny(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);
 /* Decode path stages (need topk_idx / topk_w of b200moe_route in the workspace; the fp32 intermediate [T*8, 2048] is
- * kept in the workspace's expert_out array, one row per local pair, experts ascending, tokens ascending within one).
+ * kept in the workspace's expert_out array, one row per local pair, experts ascending, tokens ascending within one;
+ * pairs without a local expert have none).
  * Replaces the reference's T = 1 path: GEMM1 with BLOCK_M = 16 (solution/python/pure_triton_impl.py:1824-1940) and
  * _t1_fused_gemm2_reduce_kernel (solution/python/pure_triton_impl.py:1676-1750). */
 int b200moe_gemv1(const b200moe_problem* p, const b200moe_workspace* ws, void* stream);
