@@ -1,12 +1,13 @@
 """GPU: the decode path (at most eight tokens) where its work split changes: one expert for all tokens, more pairs than one
 staging pass of the second kernel holds, every token on experts of its own, no local expert for some tokens; against the CPU
-oracle, and the stage entry points against the whole call."""
+oracle, the stage entry points against the whole call, the range and the precision of its sums against 64 bits."""
 import ctypes as C
 
 import pytest
 import torch
 
-from test_gpu_parity import gpu_inputs, moe, run_and_check  # noqa: F401  (fixture and helpers)
+from conftest import assert_close
+from test_gpu_parity import KEYS, gpu_inputs, moe, run_and_check  # noqa: F401  (fixture and helpers)
 
 pytestmark = pytest.mark.gpu
 
@@ -48,6 +49,22 @@ def test_decode_stages_equal_the_call(moe, T, E_local, skew):  # noqa: F811
             _lib.check(getattr(lib, "b200moe_" + stage)(C.byref(p), C.byref(ws.struct), stream), stage)
         torch.cuda.synchronize()
         assert torch.equal(out.view(T, 7168).to(torch.bfloat16), whole)
+        flat, spare = (flat16 if out.dtype == torch.bfloat16 else flat32), (0 if out.storage_offset() else -1)
+        assert flat[spare] == 3.0   # the element beside the destination
+        flat.fill_(3.0)
+
+
+@pytest.mark.parametrize("T,E_local,seed,offset,skew", [(5, 32, 14, 0, True), (1, 256, 15, 0, False), (8, 16, 14, 32, True)])
+def test_sorted_path_of_small_batches(moe, oracle, T, E_local, seed, offset, skew):  # noqa: F811
+    """At most eight tokens whose routing ran elsewhere: route, sort, gather and the token-minor GEMMs, which a routed call of
+    that size does not reach."""
+    inp = gpu_inputs(T, E_local, seed, offset, skew)
+    idx, w = moe.route(inp["routing_logits"], inp["routing_bias"], inp["routed_scaling_factor"])
+    out = moe.kernel_from_topk(idx, w, inp["hidden_states"], inp["hidden_states_scale"], inp["gemm1_weights"],
+                               inp["gemm1_weights_scale"], inp["gemm2_weights"], inp["gemm2_weights_scale"], offset)
+    moe.check_status()
+    ref = oracle.kernel(*[inp[k] for k in KEYS])
+    assert_close(out.float().cpu(), ref["out_bf16"].float(), what=f"T={T} E={E_local}")
 
 
 def layer64(inp, E_local, offset=0):

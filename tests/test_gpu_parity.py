@@ -69,9 +69,8 @@ def run_and_check(moe, oracle, T, E_local, seed, offset, skew, poison=True):
     assert torch.equal(idx, ref["topk_idx"]), "expert ids differ from the oracle"
     assert torch.equal(w, ref["topk_w"]), "routing weights differ from the oracle"
 
-    # sort metadata: bit-exact, as the forward call left it (for 2 < T <= 32 that is the fused single-launch prologue,
-    # above it the separate sort kernels).  The decode path (few expected pairs) does not sort, so the stage is run here
-    # explicitly.
+    # sort metadata: bit-exact, as the forward call left it.  The decode path (at most eight tokens) does not sort, so the
+    # stage is run here explicitly.
     from fused_moe_b200._lib import uses_decode_path
     if uses_decode_path(T, E_local):
         from fused_moe_b200 import _lib
@@ -100,21 +99,21 @@ def run_and_check(moe, oracle, T, E_local, seed, offset, skew, poison=True):
     (7, 32, 0, 0, False),      # the reference's CPU-runnable configuration
     (1, 32, 5, 96, False),     # decode path (matrix-vector kernels)
     (2, 32, 9, 0, False),      # decode path, two tokens
-    (4, 32, 14, 0, True),      # last batch size on the decode path for 32 local experts, skewed: shared experts
-    (5, 32, 14, 0, True),      # first batch size past it
-    (8, 16, 14, 32, True),     # decode path at its token limit (16 local experts)
-    (9, 8, 14, 32, True),      # nine tokens: never the decode path
-    (1, 256, 15, 0, False),    # all experts local, one token (eight pairs): fused prologue + token-minor GEMMs
-    (1, 128, 15, 64, False),   # 128 local experts: decode path for one token only
+    (4, 32, 14, 0, True),      # decode path, skewed: shared experts
+    (5, 32, 14, 0, True),      # the same router, one token more
+    (8, 16, 14, 32, True),     # largest batch on the decode path
+    (9, 8, 14, 32, True),      # first batch size on the sorted path
+    (1, 256, 15, 0, False),    # decode path, all experts local, one token (eight pairs)
+    (1, 128, 15, 64, False),   # decode path, half of the experts
     (80, 32, 1, 0, False),     # small batch
     (33, 8, 3, 60, False),     # E_local below one warp, non-zero offset, two token chunks
     (40, 3, 13, 253, True),    # last experts, skewed router
     (3, 2, 21, 100, False),    # no token reaches a local expert: all-zero output
     (300, 32, 4, 64, True),    # an expert with more than one 128-row block
     (12, 256, 6, 0, True),     # all 256 experts local: every token sums eight expert rows
-    (32, 32, 7, 32, False),    # largest batch of the fused prologue: one full token chunk
-    (31, 256, 8, 0, True),     # fused prologue, ragged chunk, every pair local (248 gathered rows)
-    (33, 32, 7, 32, False),    # first batch size on the separate route / sort / gather kernels
+    (32, 32, 7, 32, False),    # one full token chunk
+    (31, 256, 8, 0, True),     # ragged chunk, every pair local (248 gathered rows)
+    (33, 32, 7, 32, False),    # one token into the second chunk
     (112, 32, 10, 0, True),    # largest batch on the token-minor GEMMs, experts with more than one 64-row sub-block
     (113, 32, 10, 0, True),    # first batch size on the 128-token-tile GEMMs
     (256, 32, 10, 0, True),    # eight full token chunks

@@ -1,4 +1,5 @@
-"""GPU: the single-launch prologue stage (b200moe_prologue_small) leaves what route, sort and gather leave, byte for byte."""
+"""GPU: the single-launch prologue stage (b200moe_prologue_small) leaves what route, sort and gather leave, byte for byte, in
+every array that a later stage reads."""
 import ctypes as C
 
 import pytest
@@ -23,17 +24,20 @@ def test_prologue_equals_separate_stages(moe, T, E_local, skew):  # noqa: F811
                  inp["gemm2_weights"], inp["gemm2_weights_scale"], out)
     R = ws.struct.R_max
 
+    arrays = (("topk_idx", T * 8), ("topk_w", T * 8), ("chunk_bits", E_local), ("counts", E_local),
+              ("block_offsets", E_local + 1), ("total_blocks", 1), ("scatter_map", T * 8), ("sorted_token_ids", R),
+              ("sorted_weights", R), ("a_scale_sorted", 56 * R), ("a_sorted", R * 7168 // 4))
+
     def run(stages):
-        for name, n in (("a_sorted", R * 7168), ("a_scale_sorted", R * 56 * 4), ("sorted_token_ids", R * 4)):
-            ws.view(name, torch.uint8, (n,)).fill_(0x22)
+        for name, n in arrays:   # whatever a stage does not write is told from what it does
+            ws.view(name, torch.int32, (n,)).fill_(0x22222222)
         for stage in stages:
             _lib.check(getattr(lib, "b200moe_" + stage)(C.byref(p), C.byref(ws.struct), stream), stage)
         torch.cuda.synchronize()
-        arrays = (("topk_idx", T * 8), ("topk_w", T * 8), ("chunk_bits", E_local), ("counts", E_local),
-                  ("block_offsets", E_local + 1), ("total_blocks", 1), ("scatter_map", T * 8), ("sorted_token_ids", R),
-                  ("a_scale_sorted", 56 * R), ("a_sorted", R * 7168 // 4))
         return {name: ws.view(name, torch.int32, (n,)).clone() for name, n in arrays}
 
     one, three = run(("prologue_small",)), run(("route", "sort", "gather"))
     for name in one:
         assert torch.equal(one[name], three[name]), name
+    for name in ("topk_idx", "topk_w", "chunk_bits", "counts", "block_offsets", "total_blocks", "scatter_map"):
+        assert not (one[name] == 0x22222222).any(), name   # written in full
