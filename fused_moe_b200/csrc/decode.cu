@@ -19,12 +19,14 @@
 //   k_gemv2_reduce  GEMM2 and the weighted sum over experts with the same instruction.  A warp task is four output columns
 //                   for the whole batch: 8 KB of W2 per expert in registers, requested at once, the intermediate rows in
 //                   shared memory as f16 scaled per 128 columns (11-bit rounding of each element, the only one below 32
-//                   bits).  M = four columns x four quarters of K, so a warp needs no other warp's sums.
+//                   bits).  M = four columns x four quarters of K and N = the quarters of two tokens, or two columns x eight
+//                   eighths and the eighths of one token (half the shared-memory reads: 15 experts with a token each
+//                   122.5 us per call, 120.9 with it): a warp needs no other warp's sums.
 //                   With packed half FMAs and one scale per row instead, the un-rounded sums were 4.9e-4 off 64 bits, now 1.7e-4
-//                   (one 128-column block 1e6 times larger than the others: 1.3e-2, now 1.7e-4).  us of the kernel, those / now:
-//                   one to eight pairs on experts of their own 14 / 14 .. 29 / 29, 22 pairs on four hot experts 35 / 30, 64 pairs
-//                   on 25 experts 100 / 96, on 46 experts 125 / 132 (~5.1 TB/s of W2).  Refilling the registers for the next
-//                   expert piece by piece took 140 there, independent chains of instructions changed nothing.
+//                   (one 128-column block 1e6 times larger than the others: 1.3e-2, now 1.7e-4).  us per call, those / now:
+//                   T = 1 / 32 experts 22.5 / 22.7, T = 7 54.5 / 54.7, T = 8 hot experts 55.5 / 49.3, T = 8 / 256 experts 358 / 366,
+//                   hot 200 / 188, T = 2 / 256 118.7 / 120.9.  Refilling the registers for the next expert piece by piece took
+//                   7 % longer (the requests of a warp's 8 KB no longer go out together).
 // Measured: see the dispatch rule in api.cu.
 // Reference counterpart: the T = 1 path, solution/python/pure_triton_impl.py:2025-2123 (_kernel_t1) with
 // _t1_fused_gemm2_reduce_kernel (:1676-1750); oracle math solution/cuda/binding.py:157-182.
@@ -314,6 +316,7 @@ __device__ __forceinline__ void gemv2_rows(const Gemv2Shared& S, int r, int p0, 
   // Slots past the last token take whatever the next row holds (the arrays have a row more for that): an N column's sums come
   // from its own values alone, and those of such a slot are not used.
   const uint8_t* b = S.row[r - p0 + (g & 1)] + (g >> 2) * (GEMV2_STEPS * 256) + (g >> 1 & 1) * 128 + q * 32;
+  const int swap = (g >> 1 & 1) * 16;
   const float* x = &S.scale[(q >> 1) * GEMV2_STEPS][r - p0];
   float acc[P][4];
 #pragma unroll
@@ -334,7 +337,7 @@ __device__ __forceinline__ void gemv2_rows(const Gemv2Shared& S, int r, int p0, 
     for (int h = 0; h < 2; ++h) {
       uint4 bv[P];
 #pragma unroll
-      for (int p = 0; p < P; ++p) bv[p] = *reinterpret_cast<const uint4*>(b + p * (2 * G2_ROW) + i * 256 + h * 16);
+      for (int p = 0; p < P; ++p) bv[p] = *reinterpret_cast<const uint4*>(b + p * (2 * G2_ROW) + i * 256 + (h * 16 ^ swap));
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const uint2 a0 = cvt4_h2(lo[2 * h + k]), a1 = cvt4_h2(hi[2 * h + k]);
@@ -368,6 +371,47 @@ __device__ __forceinline__ void gemv2_rows(const Gemv2Shared& S, int r, int p0, 
       if (2 * p + t < n && (lane & 7) == S.L.token[r + 2 * p + t]) tot += v;
     }
   }
+}
+
+// The same for an expert with one token (`row` of the staged batch): M rows j and 8 + j: eighth j of the K columns of two of the
+// four columns, N column j: the same eighth of the token.  Eighth 2 a + b is half b of the blocks 4 a .. 4 a + 3.
+__device__ __forceinline__ void gemv2_row(const Gemv2Shared& S, int row, int token, int lane, const uint4 (&w)[4][4], float w_scale,
+                                          float& tot) {
+  const int g = lane >> 2, q = lane & 3;
+  const uint8_t* b = S.row[row] + (lane >> 3) * 1024 + (g & 1) * 128 + q * 32;
+  const int swap = (g & 1) * 16;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float c[2][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[0][j] = c[1][j] = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint4 bv = *reinterpret_cast<const uint4*>(b + i * 256 + (h * 16 ^ swap));
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const uint4 &lo = w[2 * p][i], &hi = w[2 * p + 1][i];
+          mma_k16(c[p], cvt4_h2(h ? (k ? lo.w : lo.z) : (k ? lo.y : lo.x)), cvt4_h2(h ? (k ? hi.w : hi.z) : (k ? hi.y : hi.x)),
+                  k ? bv.z : bv.x, k ? bv.w : bv.y);
+        }
+    }
+    const float f = __shfl_sync(0xffffffffu, w_scale, (lane >> 3) * 4 + i) * S.scale[q * 4 + i][row];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j] = fmaf(g & 1 ? c[j >> 1][(j & 1) * 2 + 1] : c[j >> 1][(j & 1) * 2], f, acc[j]);
+  }
+  // add the eight eighths (lanes 4 j + j / 2); afterwards lane 4 k + 9 l holds column 2 k + l
+  const bool hi = (lane & 4) != 0, odd = (lane & 8) != 0;
+  float y0 = hi ? acc[2] : acc[0], y1 = hi ? acc[3] : acc[1];
+  y0 += __shfl_xor_sync(0xffffffffu, hi ? acc[0] : acc[2], 4);
+  y1 += __shfl_xor_sync(0xffffffffu, hi ? acc[1] : acc[3], 4);
+  float z = odd ? y1 : y0;
+  z += __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 9);
+  z += __shfl_xor_sync(0xffffffffu, z, 18);
+  const float v = __shfl_sync(0xffffffffu, z, (lane >> 4) * 4 + (lane >> 3 & 1) * 9);
+  if ((lane & 7) == token) tot += v;
 }
 
 // out[t, n] = sum over the token's local experts of weight * (inter[p] . W2[e][n]).
@@ -433,7 +477,7 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             const float4 &a = v[2 * q], &b = v[2 * q + 1];
-            dst[q] = make_uint4(half2_bits(__floats2half2_rn(a.x * k, a.y * k)), half2_bits(__floats2half2_rn(a.z * k, a.w * k)),
+            dst[q ^ (c >> 2 & 1)] = make_uint4(half2_bits(__floats2half2_rn(a.x * k, a.y * k)), half2_bits(__floats2half2_rn(a.z * k, a.w * k)),
                                 half2_bits(__floats2half2_rn(b.x * k, b.y * k)), half2_bits(__floats2half2_rn(b.z * k, b.w * k)));
           }
           if ((lane & 7) == 0) S.scale[c >> 3][r] = weight * (m * (1.0f / 256.0f));
@@ -444,21 +488,31 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
       if (g >= g_end) continue;
       while (u < n_lists && L.first[u] < p1) {
         const int e = L.e[u];
-        // this lane's 64-column halves of the blocks 8 a + i of columns n0 + c and n0 + 2 + c (lane = 16 c + 8 a + 4 b + q)
-        const uint8_t* w_row = w2 + (static_cast<size_t>(e) * H + n0 + (lane >> 4)) * I + (lane >> 3 & 1) * (GEMV2_STEPS * 128) + (lane & 7) * 16;
-        uint4 w[GEMV2_STEPS][2];
-#pragma unroll
-        for (int i = 0; i < GEMV2_STEPS; ++i)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) w[i][j] = ld_stream(w_row + j * (2 * I) + i * 128);
         // lanes 0..15: the scales of the 16 K blocks
         const float w_scale = __ldg(w2_scale + (static_cast<size_t>(e) * H_BLOCKS + (n0 >> 7)) * I_BLOCKS + (lane & (I_BLOCKS - 1)));
+        const uint8_t* w_cols = w2 + (static_cast<size_t>(e) * H + n0) * I + (lane & 7) * 16;
         const int first = L.first[u], last = L.first[u + 1];
         const int r1 = last < p1 ? last : p1;
         int r = first > p0 ? first : p0;
+        if (r1 - r == 1) {
+          uint4 w[4][4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[j][i] = ld_stream(w_cols + (lane >> 3) * 512 + j * I + i * 128);
+          gemv2_row(S, r - p0, L.token[r], lane, w, w_scale, tot);
+        } else {
+          // this lane's 64-column halves of the blocks 8 a + i of columns n0 + c and n0 + 2 + c (lane = 16 c + 8 a + 4 b + q)
+          w_cols += (lane >> 4) * I + (lane >> 3 & 1) * (GEMV2_STEPS * 128);
+          uint4 w[GEMV2_STEPS][2];
+#pragma unroll
+          for (int i = 0; i < GEMV2_STEPS; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) w[i][j] = ld_stream(w_cols + j * (2 * I) + i * 128);
 #pragma unroll 1
-        for (; r + 2 < r1; r += 4) gemv2_rows<2>(S, r, p0, min(r1 - r, 4), lane, w, w_scale, tot);
-        if (r < r1) gemv2_rows<1>(S, r, p0, r1 - r, lane, w, w_scale, tot);
+          for (; r + 2 < r1; r += 4) gemv2_rows<2>(S, r, p0, min(r1 - r, 4), lane, w, w_scale, tot);
+          if (r < r1) gemv2_rows<1>(S, r, p0, r1 - r, lane, w, w_scale, tot);
+        }
         if (last > p1) break;   // the rest of this expert's tokens are in the next batch of rows
         ++u;
       }
