@@ -477,8 +477,10 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             const float4 &a = v[2 * q], &b = v[2 * q + 1];
-            dst[q ^ (c >> 2 & 1)] = make_uint4(half2_bits(__floats2half2_rn(a.x * k, a.y * k)), half2_bits(__floats2half2_rn(a.z * k, a.w * k)),
-                                half2_bits(__floats2half2_rn(b.x * k, b.y * k)), half2_bits(__floats2half2_rn(b.z * k, b.w * k)));
+            // the halves of every second 64 columns are swapped: gemv2_row reads two such pieces at a time
+            dst[q ^ (c >> 2 & 1)] =
+                make_uint4(half2_bits(__floats2half2_rn(a.x * k, a.y * k)), half2_bits(__floats2half2_rn(a.z * k, a.w * k)),
+                           half2_bits(__floats2half2_rn(b.x * k, b.y * k)), half2_bits(__floats2half2_rn(b.z * k, b.w * k)));
           }
           if ((lane & 7) == 0) S.scale[c >> 3][r] = weight * (m * (1.0f / 256.0f));
         }
@@ -489,7 +491,8 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
       while (u < n_lists && L.first[u] < p1) {
         const int e = L.e[u];
         // lanes 0..15: the scales of the 16 K blocks
-        const float w_scale = __ldg(w2_scale + (static_cast<size_t>(e) * H_BLOCKS + (n0 >> 7)) * I_BLOCKS + (lane & (I_BLOCKS - 1)));
+        const float w_scale =
+            __ldg(w2_scale + (static_cast<size_t>(e) * H_BLOCKS + (n0 >> 7)) * I_BLOCKS + (lane & (I_BLOCKS - 1)));
         const uint8_t* w_cols = w2 + (static_cast<size_t>(e) * H + n0) * I + (lane & 7) * 16;
         const int first = L.first[u], last = L.first[u + 1];
         const int r1 = last < p1 ? last : p1;
