@@ -120,11 +120,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
-// A shared-memory counter as a one-way signal: the writers add with release ordering, one reader polls it with acquire
+// A shared-memory counter as a one-way signal: the writers add to it, one reader polls it with acquire
 // loads until it reaches `target` (bounded like mbar_wait).  A poll is a plain shared-memory load: nothing parks, and
 // the reader sees the last addition a few tens of cycles after it happens.
-__device__ __forceinline__ void red_add_release_shared(uint32_t* counter, uint32_t v) {
-  asm volatile("red.release.cta.shared::cta.add.u32 [%0], %1;"
+// The addition orders nothing else (see mbar_arrive_relaxed).
+__device__ __forceinline__ void red_add_relaxed_shared(uint32_t* counter, uint32_t v) {
+  asm volatile("red.relaxed.cta.shared::cta.add.u32 [%0], %1;"
                ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(counter))), "r"(v)
                : "memory");
 }
@@ -200,6 +201,13 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const void* tmap,
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
+}
+
+// Untiled copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from this GPU's memory.
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------------------

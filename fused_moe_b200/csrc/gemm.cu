@@ -17,7 +17,11 @@
 //
 // One CTA per tile.  What paces it (cycle stamps, probes): a TMEM stage goes round MMA -> completion signal -> promotion
 // warps read it (two 64-column loads per warp) -> hand-back -> next MMA into it, and with 512 TMEM columns there are
-// only two such stages of 256 columns.  A round costs ~600 cycles of tensor work (four MMAs of 128 cycles plus issue
+// only two such stages of 256 columns.  The block scales must not come from global memory in the promotion loop: with
+// loads one chunk ahead (an L2 round trip under load is 600-900 cycles, and a releasing hand-back waits for it as well)
+// that loop was the slowest chain; through shared memory, brought by the producer, GEMM1 went 5212 -> 4915 us at T = 16384 /
+// 256 experts, 1494 -> 1316 at 14107 / 32 (hot experts), 343 -> 312 at 1500 / 64, 110 -> 103 at 333 / 32, GEMM2 unchanged.
+// A round costs ~600 cycles of tensor work (four MMAs of 128 cycles plus issue
 // gaps) and ~1100-1300 cycles of latencies (barrier wake-ups of 190-280 cycles each way, 260 for the two loads, 150 to
 // the hand-back, 170 to re-check the operands), so two stages keep the tensor pipe ~55 % busy: ~970 cycles per 128-K
 // chunk.  Things that were built, measured and did NOT move it: CTA pairs (tcgen05.mma.cta_group::2, each CTA loading
@@ -63,7 +67,10 @@ struct Cfg {
   static constexpr int STAGES = 196608 / STAGE_BYTES;  // 4 (GEMM1, 48 KB), 3 (GEMM2, 64 KB)
   static constexpr int K_CHUNKS = (MODE == 1) ? H_BLOCKS : I_BLOCKS;
   static constexpr int N_TILES = (MODE == 1) ? (I / 128) : (H / 256);  // 16, 28
+  static constexpr int W_SCALES = (MODE == 1) ? 2 * K_CHUNKS : K_CHUNKS;   // weight scales a promotion warp needs for a tile
 };
+constexpr int ROW_SCALE_BYTES = BLOCK_M * 4;   // row scales of one chunk
+constexpr int SCALE_RING = 8;                  // chunks whose row scales are kept, see GemmAux::row_scale
 
 struct TileInfo {
   int e, nt, mblk, m_local, cnt;
@@ -116,12 +123,19 @@ struct __align__(16) GemmAux {
   int off[E_GLOBAL + 1];
   int cnt[E_GLOBAL];
   float amax[2][2][BLOCK_M];
+  // Row scales, brought by the producer with the operand boxes of their chunk and covered by the same barrier.  Chunk c is
+  // requested once the MMAs of chunk c - STAGES are complete, and those were issued after every promotion warp had read
+  // chunk c - STAGES - 2, so STAGES + 2 <= SCALE_RING slots are enough.
+  alignas(16) float row_scale[SCALE_RING][BLOCK_M];
+  float w_scale[NUM_PROMO_WARPS][2 * H_BLOCKS];   // weight scales of the tile, a copy per promotion warp
   // GEMM2 epilogue: per promotion warp, 32 rows x 16 columns (+4 padding: conflict-free 16-byte accesses) through which
   // the thread-per-row accumulators are turned into stores of 64 contiguous bytes per row
   // (16-byte aligned: it is read and written with 16-byte accesses)
   alignas(16) float out_stage[NUM_PROMO_WARPS][32][20];
 };
 static_assert(offsetof(GemmAux, out_stage) % 16 == 0, "out_stage is accessed with 16-byte vectors");
+static_assert(offsetof(GemmAux, row_scale) % 16 == 0, "bulk copy destination");
+static_assert(Cfg<1>::STAGES + 2 <= SCALE_RING && Cfg<2>::STAGES + 2 <= SCALE_RING, "row scales in use");
 
 template <int MODE>
 constexpr size_t gemm_smem_bytes() {
@@ -214,7 +228,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const TileInfo ti = decode_tile(group_id, aux->off, aux->cnt, E, NT);
           for (; ahead < C::STAGES; ++ahead) {
             const uint32_t full = smem_u32(&aux->full[ahead]);
-            mbar_arrive_expect_tx(full, C::STAGE_BYTES);
+            mbar_arrive_expect_tx(full, C::STAGE_BYTES + ROW_SCALE_BYTES);
             load_weights(ti, ahead, tiles_addr + ahead * C::STAGE_BYTES + C::A_TILES * A_TILE_BYTES, full);
           }
         }
@@ -222,6 +236,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
       for (int tile = group_id; ok && tile < total_tiles; tile += num_groups) {
         const TileInfo ti = decode_tile(tile, aux->off, aux->cnt, E, NT);
+        const float* rs = args.row_scale + ti.mblk * BLOCK_M;
         for (int kb = 0; kb < C::K_CHUNKS; ++kb) {
           ok = mbar_wait(smem_u32(&aux->empty[stage]), phase ^ 1u, abort_flag, args.status, 1, kb);
           if (!ok) break;
@@ -229,7 +244,9 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const uint32_t sB = sbase + C::A_TILES * A_TILE_BYTES;
           const uint32_t full = smem_u32(&aux->full[stage]);
           const bool requested = issued < ahead;
-          if (!requested) mbar_arrive_expect_tx(full, C::STAGE_BYTES);
+          if (!requested) mbar_arrive_expect_tx(full, C::STAGE_BYTES + ROW_SCALE_BYTES);
+          bulk_load(smem_u32(&aux->row_scale[issued % SCALE_RING][0]), rs + static_cast<size_t>(kb) * args.R_max,
+                    ROW_SCALE_BYTES, full);
           tma_load_2d(sbase, &tmA, full, kb * 128, ti.mblk * BLOCK_M);
           if (MODE == 2) tma_load_2d(sbase + A_TILE_BYTES, &tmA, full, kb * 128, args.R_max + ti.mblk * BLOCK_M);
           if (!requested) load_weights(ti, kb, sB, full);
@@ -298,33 +315,35 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint32_t acc_phase = 0;
     int tile_iter = 0;
     bool ok = true;
-    // The next tile is looked up, and the scales of its first chunk are requested, before the epilogue of the current one:
-    // the look-up and the L2 round trip (~1000 cycles) then overlap the epilogue instead of delaying the first promotion.
-    // (Measured, GEMM1 / GEMM2 us: T = 14107 / 32 experts 1521 -> 1455 / 1110 -> 1073, T = 2048 / 256 1406 -> 1361 / 876 -> 853.
-    // Scales two or four chunks ahead in an unrolled loop made GEMM1 13 - 19 % slower.)
+    uint32_t chunk = 0;
+    // The next tile is looked up, and its weight scales are requested, before the epilogue of the current one, so that the
+    // look-up and the L2 round trip overlap the epilogue instead of delaying the first promotion.
     TileInfo ti = {};
-    float rs_n = 0.f, w0_n = 0.f, w1_n = 0.f;
-    const float* rs_ptr = nullptr;
-    const float* ws0_ptr = nullptr;
-    const float* ws1_ptr = nullptr;
-    auto scales_of = [&](const TileInfo& t) {
-      rs_ptr = args.row_scale + t.mblk * BLOCK_M + r_in_tile;
-      if (MODE == 1) {
-        ws0_ptr = args.w_scale + (static_cast<size_t>(t.e) * 32 + t.nt) * H_BLOCKS;
-        ws1_ptr = ws0_ptr + 16 * H_BLOCKS;
-      } else {
-        ws0_ptr = args.w_scale + (static_cast<size_t>(t.e) * H_BLOCKS + t.nt * 2 + h) * I_BLOCKS;
-        ws1_ptr = ws0_ptr;
+    // Weight scales of tile `ti`: GEMM1 W1 scales then W3 scales (16 blocks on), GEMM2 those of this warp's 128 columns.
+    // Each lane requests its share into registers; keep_scales() puts them into this warp's shared-memory copy.
+    float w_next[(C::W_SCALES + 31) / 32];
+    float* w_own = aux->w_scale[warp];
+    auto request_scales = [&]() {
+      const float* src = args.w_scale + ((MODE == 1) ? (static_cast<size_t>(ti.e) * 32 + ti.nt) * H_BLOCKS
+                                                     : (static_cast<size_t>(ti.e) * H_BLOCKS + ti.nt * 2 + h) * I_BLOCKS);
+#pragma unroll
+      for (int i = 0; i < (C::W_SCALES + 31) / 32; ++i) {
+        const int j = i * 32 + lane;
+        if (j < C::W_SCALES) w_next[i] = __ldg(src + j + ((MODE == 1 && j >= H_BLOCKS) ? 15 * H_BLOCKS : 0));
       }
-      rs_n = __ldg(rs_ptr);
-      w0_n = __ldg(ws0_ptr);
-      w1_n = __ldg(ws1_ptr);
+    };
+    auto keep_scales = [&]() {
+#pragma unroll
+      for (int i = 0; i < (C::W_SCALES + 31) / 32; ++i)
+        if (i * 32 + lane < C::W_SCALES) w_own[i * 32 + lane] = w_next[i];
+      __syncwarp();
     };
     if (group_id < total_tiles) {
       ti = decode_tile(group_id, aux->off, aux->cnt, E, NT);
-      scales_of(ti);
+      request_scales();
     }
     for (int tile = group_id; ok && tile < total_tiles; tile += num_groups, ++tile_iter) {
+      keep_scales();
       // 128 fp32 accumulators per thread, kept as 64 pairs so the promotion runs on the packed FMA (2 lanes / issue)
       float2 acc2[64];
 #pragma unroll
@@ -332,16 +351,13 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #define ACC(j) (((j) & 1) ? acc2[(j) >> 1].y : acc2[(j) >> 1].x)
 
       for (int kb = 0; kb < C::K_CHUNKS; ++kb) {
-        const float sc0 = rs_n * w0_n;
-        const float sc1 = rs_n * w1_n;
-        if (kb + 1 < C::K_CHUNKS) {
-          rs_n = __ldg(rs_ptr + static_cast<size_t>(kb + 1) * args.R_max);
-          w0_n = __ldg(ws0_ptr + kb + 1);
-          w1_n = __ldg(ws1_ptr + kb + 1);
-        }
         ok = mbar_wait_all(smem_u32(&aux->tfull[acc]), acc_phase, abort_flag, args.status, 4, kb);
         if (!ok) break;
         tc_fence_after();
+        const float rs = aux->row_scale[chunk % SCALE_RING][r_in_tile];
+        const float sc0 = rs * w_own[kb];
+        const float sc1 = (MODE == 1) ? rs * w_own[C::K_CHUNKS + kb] : sc0;
+        ++chunk;
         const uint32_t taddr = tmem_base + static_cast<uint32_t>(acc * TILE_N) + (static_cast<uint32_t>(q * 32) << 16);
         // This warp's 128 accumulators are two runs of 64 TMEM columns — MODE 1: [64h, 64h+64) holds W1 ("up") and
         // [128+64h, 128+64h+64) holds W3 ("gate"); MODE 2: [128h, 128h+128) — each read with one 64-column load
@@ -357,7 +373,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // all of this warp's reads of the stage are complete (tcgen05.wait::ld is warp-synchronous): hand it back
             // to the MMA issuer
             tc_fence_before();
-            if (lane == 0) red_add_release_shared(&aux->drained[acc], 1u);
+            if (lane == 0) red_add_relaxed_shared(&aux->drained[acc], 1u);
           }
           const float2 sc2 = make_float2(sc, sc);
 #pragma unroll
@@ -374,7 +390,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const bool valid = (done.m_local * BLOCK_M + r_in_tile) < done.cnt;
       if (tile + num_groups < total_tiles) {
         ti = decode_tile_from(tile + num_groups, done.e, aux->off, aux->cnt, NT);
-        scales_of(ti);
+        request_scales();
       }
 
       if (MODE == 1) {
