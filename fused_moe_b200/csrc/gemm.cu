@@ -29,8 +29,8 @@
 // a second MMA-issuing thread (one per TMEM stage; with it the issuer has slack and the promotion warps are busy
 // ~850 of every ~980 cycles: wake-up, 64-column load, 32 packed FMAs, load, 32 FMAs, nothing overlapped because 128
 // accumulators + 64 loaded values fill the 232 registers), the last promotion warp issuing the next MMAs itself (the
-// issue of four MMAs blocks its thread for ~430 cycles: 38 % slower), parking barrier polls with a suspend-time hint,
-// and a relaxed instead of a releasing hand-back.  The hand-back itself is a shared-memory counter polled by the
+// issue of four MMAs blocks its thread for ~430 cycles: 38 % slower), and parking barrier polls with a suspend-time hint.
+// The hand-back itself is a shared-memory counter polled by the
 // issuer (2-7 % faster than an mbarrier).  In isolation the pieces run at 512 (MMA), 320 (promotion, 8 warps) and
 // 610-690 (48 KB of loads per SM from L2, all SMs) cycles per chunk, and ~600 when all three run unsynchronised.
 //
