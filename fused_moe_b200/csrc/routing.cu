@@ -194,28 +194,43 @@ k_small_prologue(const float* __restrict__ logits, const uint16_t* __restrict__ 
   }
 }
 
-// chunk_bits from an existing topk_idx: a CTA per 32-token chunk, a thread per (token, k) pair, the words put together in
-// shared memory.  (One warp per chunk, whose lanes held 256-bit masks that 256 ballots transposed, took 9.1 us for
-// 16384 tokens / 256 experts, now 3.3; 1500 / 64 3.9 -> 3.3.)
-__global__ void __launch_bounds__(32 * TOP_K)
-k_topk_bits(const int* __restrict__ topk_idx, long long idx_stride, int T, int local_offset, int E_local,
+// chunk_bits from an existing topk_idx: one warp per 32-token chunk, lane = token.
+__global__ void __launch_bounds__(128)
+k_topk_bits(const int* __restrict__ topk_idx, long long idx_stride, int T, int local_offset, int E_local, int n_chunks,
             uint32_t* __restrict__ chunk_bits, const b200moe_ep_plan* __restrict__ plan) {
-  static_assert(32 * TOP_K >= E_GLOBAL, "a thread per word");
-  __shared__ uint32_t s_bits[E_GLOBAL];
-  const int chunk = blockIdx.x;
-  const int lane = threadIdx.x / TOP_K;   // token of the chunk
+  const int lane = threadIdx.x & 31;
+  const int chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   pdl_launch_dependents();
-  if (threadIdx.x < E_GLOBAL) s_bits[threadIdx.x] = 0;
   pdl_wait();
-  __syncthreads();
+  if (chunk >= n_chunks) return;
   if (plan) T = min(T, plan->n_recv);   // rows past the received count hold stale records: they select nothing
   const int t = chunk * 32 + lane;
+  uint32_t mask[E_GLOBAL / 32];
+#pragma unroll
+  for (int i = 0; i < E_GLOBAL / 32; ++i) mask[i] = 0;
   if (t < T) {
-    const int le = __ldg(topk_idx + static_cast<size_t>(t) * idx_stride + threadIdx.x % TOP_K) - local_offset;
-    if (le >= 0 && le < E_local) atomicOr(&s_bits[le], 1u << lane);
+#pragma unroll
+    for (int k = 0; k < TOP_K; ++k) {
+      int le = __ldg(topk_idx + static_cast<size_t>(t) * idx_stride + k) - local_offset;
+      if (le >= 0 && le < E_local) {
+#pragma unroll
+        for (int i = 0; i < E_GLOBAL / 32; ++i)
+          if (i == (le >> 5)) mask[i] |= 1u << (le & 31);
+      }
+    }
   }
-  __syncthreads();
-  if (threadIdx.x < E_local) chunk_bits[static_cast<size_t>(chunk) * E_local + threadIdx.x] = s_bits[threadIdx.x];
+#pragma unroll
+  for (int i = 0; i < E_GLOBAL / 32; ++i) {
+    if (i * 32 >= E_local) break;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      uint32_t w = __ballot_sync(0xffffffffu, (mask[i] >> j) & 1u);
+      if (lane == j) mine = w;
+    }
+    int e = i * 32 + lane;
+    if (e < E_local) chunk_bits[static_cast<size_t>(chunk) * E_local + e] = mine;
+  }
 }
 
 int launch_route(const b200moe_problem* p, const b200moe_workspace* ws, cudaStream_t st) {
@@ -252,10 +267,11 @@ int launch_small_prologue(const b200moe_problem* p, const b200moe_workspace* ws,
 
 int launch_topk_bits(const b200moe_problem* p, const b200moe_workspace* ws, cudaStream_t st) {
   if (p->T == 0) return B200MOE_OK;
+  int grid = (ws->n_chunks + 3) / 4;
   const int* idx = p->routing_logits ? ws->topk_idx : p->topk_idx_in;
-  B200MOE_CUDA_TRY(launch_pdl(k_topk_bits, dim3(ws->n_chunks), dim3(32 * TOP_K), 0, st, idx,
+  B200MOE_CUDA_TRY(launch_pdl(k_topk_bits, dim3(grid), dim3(128), 0, st, idx,
                               p->topk_row_stride ? p->topk_row_stride : static_cast<long long>(TOP_K), p->T, p->local_expert_offset, p->E_local,
-                              ws->chunk_bits, p->plan));
+                              ws->n_chunks, ws->chunk_bits, p->plan));
   return B200MOE_OK;
 }
 
