@@ -84,6 +84,19 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 #endif
   return ok;
 }
+// One look at a barrier phase that never parks the thread.  Its result takes ~110 cycles even when the phase has long been
+// complete, so a caller that can asks early and uses the answer later.
+__device__ __forceinline__ uint32_t mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok;
+}
 // Wait on an mbarrier phase with a time limit.  Returns false (and records why) instead of hanging: `abort_flag` is a
 // CTA-shared word every waiting role looks at between polls, so one role giving up releases the others within one poll
 // period.  The limit is counted on the SM's cycle counter, read only when a poll came back empty, so a healthy wait
@@ -144,6 +157,46 @@ __device__ __forceinline__ bool counter_wait(const uint32_t* counter, uint32_t t
   uint32_t spins = 0;
   for (;;) {
     if (ld_acquire_shared(counter) >= target) return true;
+    if ((++spins & 0xffu) == 0) {
+      if (*abort_flag) return false;
+      const long long now = clock64();
+      if (t0 == 0) {
+        t0 = now;
+      } else if (now - t0 > WAIT_LIMIT_CYCLES) {
+        *abort_flag = 1;
+        if (atomicCAS(status, ST_OK, ST_WAIT_TIMEOUT) == ST_OK) {
+          status[1] = static_cast<int>(blockIdx.x);
+          status[2] = role;
+          status[3] = detail;
+        }
+        return false;
+      }
+    }
+  }
+}
+
+// Eight one-byte counters in shared memory as a one-way signal: each of eight writers stores its own running count (modulo
+// 256) with a plain store that orders nothing else (see mbar_arrive_relaxed), one reader polls the word until all of them
+// show `target` (bounded like mbar_wait).  No writer may run past `target` before the reader has seen it.
+__device__ __forceinline__ void st_relaxed_shared_u8(uint8_t* p, uint32_t v) {
+  asm volatile("st.relaxed.cta.shared::cta.u8 [%0], %1;"
+               ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(v)
+               : "memory");
+}
+__device__ __forceinline__ bool flags_equal(uint32_t flags8, uint32_t target4) {
+  uint32_t a, b;
+  asm volatile("ld.volatile.shared::cta.v2.u32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(flags8) : "memory");
+  return ((a ^ target4) | (b ^ target4)) == 0;
+}
+__device__ __forceinline__ bool flags_wait(const uint8_t* flags, uint32_t target, volatile int* abort_flag, int* status,
+                                           int role, int detail) {
+  const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(flags));
+  const uint32_t target4 = (target & 0xffu) * 0x01010101u;
+  if (flags_equal(addr, target4)) return true;
+  long long t0 = 0;
+  uint32_t spins = 0;
+  for (;;) {
+    if (flags_equal(addr, target4)) return true;
     if ((++spins & 0xffu) == 0) {
       if (*abort_flag) return false;
       const long long now = clock64();
@@ -244,6 +297,16 @@ __device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t a_desc, uint
       : "memory");
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// The same, naming the loaded registers: what uses them cannot be scheduled above the wait.
+#define B200MOE_RW8(r, i) "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7])
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&a)[32], uint32_t (&b)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : B200MOE_RW8(a, 0), B200MOE_RW8(a, 8), B200MOE_RW8(a, 16), B200MOE_RW8(a, 24),
+                 B200MOE_RW8(b, 0), B200MOE_RW8(b, 8), B200MOE_RW8(b, 16), B200MOE_RW8(b, 24)
+               :
+               : "memory");
+}
+#undef B200MOE_RW8
 
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp receives lane (base+i), r[j] = column (col0+j).
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {

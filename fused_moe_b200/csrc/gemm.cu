@@ -21,6 +21,10 @@
 // loads one chunk ahead (an L2 round trip under load is 600-900 cycles, and a releasing hand-back waits for it as well)
 // that loop was the slowest chain; through shared memory, brought by the producer, GEMM1 went 5212 -> 4915 us at T = 16384 /
 // 256 experts, 1494 -> 1316 at 14107 / 32 (hot experts), 343 -> 312 at 1500 / 64, 110 -> 103 at 333 / 32, GEMM2 unchanged.
+// GEMM2's loop also spends fewer synchronisations per chunk (one commit, a hand-back byte per warp, barrier looks asked for
+// early, 32-column loads in pairs; a look at a barrier takes ~110 cycles even if it is long complete, a shared-memory
+// atomic 110, a second commit 130): 4225 -> 4122 us at T = 16384 / 256, 1094 -> 1064 at 14107 / 32 (hot experts), 340 -> 332
+// at 4096 / 32 (hot experts), 240 -> 237 at 1500 / 64.  The same in GEMM1 made it 4-7 % SLOWER at T >= 4096, so it keeps its form.
 // A round costs ~600 cycles of tensor work (four MMAs of 128 cycles plus issue
 // gaps) and ~1100-1300 cycles of latencies (barrier wake-ups of 190-280 cycles each way, 260 for the two loads, 150 to
 // the hand-back, 170 to re-check the operands), so two stages keep the tensor pipe ~55 % busy: ~970 cycles per 128-K
@@ -120,6 +124,7 @@ struct __align__(16) GemmAux {
   // per TMEM stage: promotion warps that have finished reading it, counted up for ever (8 per fill).  The MMA issuer
   // polls it with plain loads; an mbarrier hand-back measured 2-7 % slower (the issuer's wake-up is on its serial path)
   uint32_t drained[2];
+  alignas(8) uint8_t handed[2][NUM_PROMO_WARPS];   // GEMM2's form of the same: a count (modulo 256) per promotion warp
   int off[E_GLOBAL + 1];
   int cnt[E_GLOBAL];
   float amax[2][2][BLOCK_M];
@@ -134,12 +139,22 @@ struct __align__(16) GemmAux {
   alignas(16) float out_stage[NUM_PROMO_WARPS][32][20];
 };
 static_assert(offsetof(GemmAux, out_stage) % 16 == 0, "out_stage is accessed with 16-byte vectors");
+static_assert(NUM_PROMO_WARPS == 8, "one byte each of the word the issuer polls");
+static_assert(Cfg<2>::K_CHUNKS % 2 == 0, "a tile's first chunk goes to TMEM stage 0");
 static_assert(offsetof(GemmAux, row_scale) % 16 == 0, "bulk copy destination");
 static_assert(Cfg<1>::STAGES + 2 <= SCALE_RING && Cfg<2>::STAGES + 2 <= SCALE_RING, "row scales in use");
 
 template <int MODE>
 constexpr size_t gemm_smem_bytes() {
   return 1024 + static_cast<size_t>(Cfg<MODE>::STAGES) * Cfg<MODE>::STAGE_BYTES + sizeof(GemmAux);
+}
+
+// 16 pairs of sums += 32 TMEM values x their scale, on the packed FMA.
+__device__ __forceinline__ void fold(float2* sums, const uint32_t (&t)[32], float scale) {
+  const float2 s2 = make_float2(scale, scale);
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    sums[j] = __ffma2_rn(make_float2(__uint_as_float(t[2 * j]), __uint_as_float(t[2 * j + 1])), s2, sums[j]);
 }
 
 template <int MODE>
@@ -165,6 +180,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     aux->drained[0] = 0;
     aux->drained[1] = 0;
   }
+  if (threadIdx.x < 2 * NUM_PROMO_WARPS) (&aux->handed[0][0])[threadIdx.x] = 0;
 
   if (warp == PRODUCER_WARP && lane == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -273,6 +289,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       int stage = 0, acc = 0;
       uint32_t phase = 0;
       uint32_t chunk = 0;                // chunks issued so far: chunk c is fill number c / 2 of TMEM stage c % 2
+      uint32_t landed = 0;               // GEMM2: the next chunk's operands, as seen once the current one had been issued
       bool ok = true;
       for (int tile = group_id; ok && tile < total_tiles; tile += num_groups) {
         for (int kb = 0; kb < C::K_CHUNKS; ++kb) {
@@ -282,9 +299,12 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const uint32_t d = tmem_base + static_cast<uint32_t>(acc * TILE_N);
           const uint64_t a0 = umma_desc_sw128(sbase);
           const uint64_t b0 = umma_desc_sw128(sbase + C::A_TILES * A_TILE_BYTES);
-          ok = mbar_wait(smem_u32(&aux->full[stage]), phase, abort_flag, args.status, 3, kb);
+          if (MODE == 1 || !landed) ok = mbar_wait(smem_u32(&aux->full[stage]), phase, abort_flag, args.status, 3, kb);
           if (!ok) break;
-          ok = counter_wait(&aux->drained[acc], (chunk >> 1) * NUM_PROMO_WARPS, abort_flag, args.status, 2, kb);
+          if (MODE == 1)
+            ok = counter_wait(&aux->drained[acc], (chunk >> 1) * NUM_PROMO_WARPS, abort_flag, args.status, 2, kb);
+          else
+            ok = flags_wait(aux->handed[acc], chunk >> 1, abort_flag, args.status, 2, kb);
           if (!ok) break;
           ++chunk;
           tc_fence_after();
@@ -296,8 +316,12 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int k4 = 0; k4 < 4; ++k4) tc_mma_f8(d, a1 + 2 * k4, b0 + 2 * k4, IDESC, 1u);
           }
           tc_commit(smem_u32(&aux->empty[stage]));
-          tc_commit(smem_u32(&aux->tfull[acc]));
+          // GEMM2's promotion warps wait for `empty` too: one commit (70 cycles of this thread, a second one 130) says both
+          // that the operands may be overwritten and that the sums are in TMEM.  Its phase cannot run ahead of a waiter:
+          // chunk c + STAGES is issued only after chunk c + STAGES - 2 >= c has left TMEM.
+          if (MODE == 1) tc_commit(smem_u32(&aux->tfull[acc]));
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
+          if (MODE == 2) landed = mbar_test(smem_u32(&aux->full[stage]), phase);
           acc ^= 1;
         }
       }
@@ -316,6 +340,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     int tile_iter = 0;
     bool ok = true;
     uint32_t chunk = 0;
+    bool arrived = false;   // GEMM2: the next chunk's barrier, as seen while the current one was folded in
     // The next tile is looked up, and its weight scales are requested, before the epilogue of the current one, so that the
     // look-up and the L2 round trip overlap the epilogue instead of delaying the first promotion.
     TileInfo ti = {};
@@ -350,22 +375,53 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       for (int j = 0; j < 64; ++j) acc2[j] = make_float2(0.f, 0.f);
 #define ACC(j) (((j) & 1) ? acc2[(j) >> 1].y : acc2[(j) >> 1].x)
 
-      for (int kb = 0; kb < C::K_CHUNKS; ++kb) {
+      if (MODE == 2) {
+        int stage = static_cast<int>(chunk % C::STAGES);
+        uint32_t phase = (chunk / C::STAGES) & 1u;
+        for (int kb = 0; kb < C::K_CHUNKS; ++kb, ++chunk) {
+          if (!arrived) ok = mbar_wait_all(smem_u32(&aux->empty[stage]), phase, abort_flag, args.status, 4, kb);
+          if (!ok) break;
+          tc_fence_after();
+          const float sc = aux->row_scale[chunk % SCALE_RING][r_in_tile] * w_own[kb];
+          // 128 columns in four loads of 32 (75 cycles each for one warp): the first two together, the third and fourth
+          // while the first two are folded in.  96 loaded values and 128 sums are as many registers as a thread can have.
+          const uint32_t taddr = tmem_base + static_cast<uint32_t>((kb & 1) * TILE_N + h * 128) +
+                                 (static_cast<uint32_t>(q * 32) << 16);
+          uint32_t t0[32], t1[32], t2[32], t3[32];
+          tmem_ld32(taddr, t0);
+          tmem_ld32(taddr + 32, t1);
+          tc_wait_ld(t0, t1);
+          tmem_ld32(taddr + 64, t2);
+          fold(acc2, t0, sc);
+          tmem_ld32(taddr + 96, t3);
+          fold(acc2 + 16, t1, sc);
+          tc_wait_ld(t2, t3);
+          // this warp has read its part of the stage (tcgen05.wait::ld is warp-synchronous): hand it back, and ask for the
+          // next chunk's barrier before folding the rest in
+          tc_fence_before();
+          if (lane == 0) st_relaxed_shared_u8(&aux->handed[kb & 1][warp], chunk / 2 + 1);
+          if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
+          const uint32_t next = mbar_test(smem_u32(&aux->empty[stage]), phase);
+          fold(acc2 + 32, t2, sc);
+          fold(acc2 + 48, t3, sc);
+          arrived = __all_sync(0xffffffffu, next);
+        }
+      }
+      for (int kb = 0; MODE == 1 && kb < C::K_CHUNKS; ++kb) {
         ok = mbar_wait_all(smem_u32(&aux->tfull[acc]), acc_phase, abort_flag, args.status, 4, kb);
         if (!ok) break;
         tc_fence_after();
         const float rs = aux->row_scale[chunk % SCALE_RING][r_in_tile];
         const float sc0 = rs * w_own[kb];
-        const float sc1 = (MODE == 1) ? rs * w_own[C::K_CHUNKS + kb] : sc0;
+        const float sc1 = rs * w_own[(MODE == 1 ? C::K_CHUNKS : 0) + kb];
         ++chunk;
         const uint32_t taddr = tmem_base + static_cast<uint32_t>(acc * TILE_N) + (static_cast<uint32_t>(q * 32) << 16);
-        // This warp's 128 accumulators are two runs of 64 TMEM columns — MODE 1: [64h, 64h+64) holds W1 ("up") and
-        // [128+64h, 128+64h+64) holds W3 ("gate"); MODE 2: [128h, 128h+128) — each read with one 64-column load
-        // (fewer, wider loads measured faster than four 32-column loads, pipelined or not).
+        // This warp's 128 accumulators are two runs of 64 TMEM columns: [64h, 64h+64) holds W1 ("up") and
+        // [128+64h, 128+64h+64) holds W3 ("gate"), each read with one 64-column load.
 #pragma unroll
         for (int run = 0; run < 2; ++run) {
-          const uint32_t col = static_cast<uint32_t>((MODE == 1) ? (run * 128 + h * 64) : (h * 128 + run * 64));
-          const float sc = (MODE == 1 && run == 1) ? sc1 : sc0;
+          const uint32_t col = static_cast<uint32_t>(run * 128 + h * 64);
+          const float sc = run == 1 ? sc1 : sc0;
           uint32_t tmp[64];
           tmem_ld64(taddr + col, tmp);
           tc_wait_ld();
