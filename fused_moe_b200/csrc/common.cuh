@@ -378,8 +378,54 @@ __device__ __forceinline__ float bf16_bits_to_float(uint16_t b) { return __uint_
 // Programmatic dependent launch: every kernel of the layer lets its successor be scheduled early
 // (pdl_launch_dependents at entry) and blocks in pdl_wait until its predecessor has completed and flushed before it
 // touches global memory.  Only launch latency and per-CTA set-up overlap; data dependences stay kernel-to-kernel.
+//
+// A kernel is therefore resident while earlier ones, back to the call before or a foreign kernel in front of it, are still
+// writing what it will read: nothing in global memory is read-only for its lifetime.  `const __restrict__` and __ldg say it
+// is; the compiler may then take a load for invariant and move it above the wait (a "memory" clobber does not hold a load
+// through an unaliased pointer), and the non-coherent path need not see what was written meanwhile.  So no pointer to global
+// memory is declared __restrict__ and every kernel loads with ld_dep() or ld_l2(): volatile like the wait, which they
+// cannot pass, and coherent.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Load below pdl_wait().  No "memory" clobber: loads in a row may all be in flight, but one written behind a store waits for it
+// in the instruction stream, so load a batch into registers first.
+template <typename T>
+__device__ __forceinline__ T ld_dep(const T* p) {
+  static_assert(sizeof(T) == 1 || sizeof(T) == 2 || sizeof(T) == 4 || sizeof(T) == 16, "widths in use");
+  if constexpr (sizeof(T) == 16) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return *reinterpret_cast<T*>(&v);
+  } else if constexpr (sizeof(T) == 4) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return *reinterpret_cast<T*>(&v);
+  } else if constexpr (sizeof(T) == 2) {
+    uint16_t v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return *reinterpret_cast<T*>(&v);
+  } else {
+    uint32_t v;
+    asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
+    return static_cast<T>(v);
+  }
+}
+// The same from L2, past this SM's L1: for words read before the kernel's own wait (the sort metadata of an early GEMM, complete
+// since the release that let the kernel start), for the expert-parallel plan, and for what other CTAs of the kernel wrote.
+template <typename T>
+__device__ __forceinline__ T ld_l2(const T* p) {
+  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "widths in use");
+  if constexpr (sizeof(T) == 8) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return *reinterpret_cast<T*>(&v);
+  } else {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return *reinterpret_cast<T*>(&v);
+  }
+}
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
@@ -405,5 +451,19 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   } while (0)
 
 int record_cuda_error(cudaError_t e);
+
+// One 7168-byte row, global to global, by a warp: half of a lane's 14 pieces in registers at a time (see ld_dep).
+__device__ __forceinline__ void copy_row(uint8_t* dst, const uint8_t* src, int lane) {
+  constexpr int PIECES = H / 16 / 32, BATCH = PIECES / 2;
+  static_assert(PIECES * 16 * 32 == H && BATCH * 2 == PIECES, "whole pieces and batches");
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    uint4 v[BATCH];
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) v[i] = ld_dep(reinterpret_cast<const uint4*>(src) + (b * BATCH + i) * 32 + lane);
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) reinterpret_cast<uint4*>(dst)[(b * BATCH + i) * 32 + lane] = v[i];
+  }
+}
 
 }  // namespace b200moe

@@ -42,10 +42,10 @@ constexpr int DEC_PAIRS = DEC_T * TOP_K;
 constexpr int DEC_N = 8;                                // tokens of one list = N of the instruction
 static_assert(DEC_T <= DEC_N, "an expert's tokens are one N tile, and one lane each in GEMV2's sums");
 
-// streaming 16-byte load: weights are read once, keep them out of L1
+// streaming 16-byte load (see ld_dep): weights are read once, keep them out of L1
 __device__ __forceinline__ uint4 ld_stream(const uint8_t* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;
@@ -144,11 +144,11 @@ static size_t gemv1_smem(int T) { return sizeof(Gemv1Shared) + 16 + static_cast<
 
 template <bool ROUTE>
 __global__ void __launch_bounds__(G1_THREADS, 1)
-k_gemv1_swiglu(const float* __restrict__ logits, const uint16_t* __restrict__ bias, float scale_factor,
-               int* __restrict__ topk_idx, float* __restrict__ topk_w, uint32_t* __restrict__ chunk_bits,
-               const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, int T, int local_offset,
-               int E_local, const uint8_t* __restrict__ w13, const float* __restrict__ w13_scale,
-               const uint8_t* __restrict__ w2, float* __restrict__ inter) {
+k_gemv1_swiglu(const float* logits, const uint16_t* bias, float scale_factor,
+               int* topk_idx, float* topk_w, uint32_t* chunk_bits,
+               const uint8_t* hidden, const float* hidden_scale, int T, int local_offset,
+               int E_local, const uint8_t* w13, const float* w13_scale,
+               const uint8_t* w2, float* inter) {
   extern __shared__ __align__(16) uint8_t dyn[];
   uint8_t* rows = dyn;                                        // [T][G1_ROW]
   Gemv1Shared& S = *reinterpret_cast<Gemv1Shared*>(dyn + static_cast<size_t>(T) * G1_ROW);
@@ -159,7 +159,7 @@ k_gemv1_swiglu(const float* __restrict__ logits, const uint16_t* __restrict__ bi
   pdl_launch_dependents();
   for (int c = threadIdx.x; c < T * (H / 16); c += G1_THREADS) {
     const int t = c / (H / 16), u = c - t * (H / 16);
-    const uint4 h = __ldg(reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(t) * H) + u);
+    const uint4 h = ld_dep(reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(t) * H) + u);
     const uint2 h0 = cvt4_h2(h.x), h1 = cvt4_h2(h.y), h2 = cvt4_h2(h.z), h3 = cvt4_h2(h.w);
     uint4* dst = reinterpret_cast<uint4*>(rows + t * G1_ROW + u * 32);
     dst[0] = make_uint4(h0.x, h0.y, h1.x, h1.y);
@@ -167,7 +167,7 @@ k_gemv1_swiglu(const float* __restrict__ logits, const uint16_t* __restrict__ bi
   }
   for (int c = threadIdx.x; c < T * H_BLOCKS; c += G1_THREADS) {
     const int kb = c / T, t = c - kb * T;
-    S.scale[t * G1_SCALES + kb] = __ldg(hidden_scale + c);
+    S.scale[t * G1_SCALES + kb] = ld_dep(hidden_scale + c);
   }
   __syncthreads();   // masks are zero
   for (int t = warp; t < T; t += G1_TEAMS * G1_TEAM_WARPS) {
@@ -180,7 +180,7 @@ k_gemv1_swiglu(const float* __restrict__ logits, const uint16_t* __restrict__ bi
         topk_w[t * TOP_K + lane] = w;
       }
     } else if (lane < TOP_K) {
-      idx = topk_idx[t * TOP_K + lane];
+      idx = ld_dep(topk_idx + t * TOP_K + lane);
     }
     const int le = idx - local_offset;
     if (lane < TOP_K && le >= 0 && le < E_local) atomicOr(&L.mask[le], 1u << t);
@@ -205,7 +205,7 @@ k_gemv1_swiglu(const float* __restrict__ logits, const uint16_t* __restrict__ bi
   // lanes 0..7: scales of W1 for the warp's eight blocks, lanes 8..15: of W3
   auto task_scale = [&](int task) {
     const int u = task / TASKS_PER_LIST, n0 = (task - u * TASKS_PER_LIST) * G1_COLS;
-    return __ldg(w13_scale + (static_cast<size_t>(L.e[u]) * 32 + (lane & 8) * 2 + (n0 >> 7)) * H_BLOCKS + (lane & 7) * G1_TEAM_WARPS + wt);
+    return ld_dep(w13_scale + (static_cast<size_t>(L.e[u]) * 32 + (lane & 8) * 2 + (n0 >> 7)) * H_BLOCKS + (lane & 7) * G1_TEAM_WARPS + wt);
   };
   uint4 ring[4][4];
   auto load = [&](uint4 (&s)[4], const uint8_t* p) {
@@ -416,9 +416,9 @@ __device__ __forceinline__ void gemv2_row(const Gemv2Shared& S, int row, int tok
 
 // out[t, n] = sum over the token's local experts of weight * (inter[p] . W2[e][n]).
 __global__ void __launch_bounds__(G2_THREADS, 1)
-k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx, const float* __restrict__ topk_w,
-               int T, int local_offset, int E_local, const uint8_t* __restrict__ w2, const float* __restrict__ w2_scale,
-               uint16_t* __restrict__ out, float* __restrict__ out_f32) {
+k_gemv2_reduce(const float* inter, const int* topk_idx, const float* topk_w,
+               int T, int local_offset, int E_local, const uint8_t* w2, const float* w2_scale,
+               uint16_t* out, float* out_f32) {
   extern __shared__ __align__(16) uint8_t dyn[];
   Gemv2Shared& S = *reinterpret_cast<Gemv2Shared*>(dyn);
   ExpertLists& L = S.L;
@@ -429,7 +429,7 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
   pdl_wait();
   __syncthreads();
   if (threadIdx.x < T * TOP_K) {
-    const int le = __ldg(topk_idx + threadIdx.x) - local_offset;
+    const int le = ld_dep(topk_idx + threadIdx.x) - local_offset;
     if (le >= 0 && le < E_local) atomicOr(&L.mask[le], 1u << (threadIdx.x / TOP_K));
   }
   __syncthreads();
@@ -458,13 +458,13 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
           const float4* x = reinterpret_cast<const float4*>(inter + static_cast<size_t>(p0 + r) * I) + c * 4;
           float4 v[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) v[q] = __ldg(x + q);
+          for (int q = 0; q < 4; ++q) v[q] = ld_dep(x + q);
           // the routing weight: the slot in which the pair's token holds the pair's expert
           int u_r = 0;
           while (L.first[u_r + 1] <= p0 + r) ++u_r;
           const int at = L.token[p0 + r] * TOP_K + (lane & (TOP_K - 1));
-          const float wk = __ldg(topk_w + at);
-          const uint32_t hit = __ballot_sync(0xffffffffu, __ldg(topk_idx + at) == L.e[u_r] + local_offset);
+          const float wk = ld_dep(topk_w + at);
+          const uint32_t hit = __ballot_sync(0xffffffffu, ld_dep(topk_idx + at) == L.e[u_r] + local_offset);
           const float weight = __shfl_sync(0xffffffffu, wk, __ffs(hit) - 1);
           float m = 1e-36f;   // 256 / m stays finite
 #pragma unroll
@@ -492,7 +492,7 @@ k_gemv2_reduce(const float* __restrict__ inter, const int* __restrict__ topk_idx
         const int e = L.e[u];
         // lanes 0..15: the scales of the 16 K blocks
         const float w_scale =
-            __ldg(w2_scale + (static_cast<size_t>(e) * H_BLOCKS + (n0 >> 7)) * I_BLOCKS + (lane & (I_BLOCKS - 1)));
+            ld_dep(w2_scale + (static_cast<size_t>(e) * H_BLOCKS + (n0 >> 7)) * I_BLOCKS + (lane & (I_BLOCKS - 1)));
         const uint8_t* w_cols = w2 + (static_cast<size_t>(e) * H + n0) * I + (lane & 7) * 16;
         const int first = L.first[u], last = L.first[u + 1];
         const int r1 = last < p1 ? last : p1;

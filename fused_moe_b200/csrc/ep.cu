@@ -22,8 +22,8 @@ int launch_combine_half(const void* rows, const int* slot_map, int T, uint16_t* 
 
 // chunk_bits over destination ranks: one warp per 32-token chunk, lane = token.
 __global__ void __launch_bounds__(128)
-k_dest_bits(const int* __restrict__ topk_idx, int T, int experts_per_rank, int world, int n_chunks,
-            uint32_t* __restrict__ chunk_bits) {
+k_dest_bits(const int* topk_idx, int T, int experts_per_rank, int world, int n_chunks,
+            uint32_t* chunk_bits) {
   const int lane = threadIdx.x & 31;
   const int chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   pdl_launch_dependents();
@@ -36,7 +36,7 @@ k_dest_bits(const int* __restrict__ topk_idx, int T, int experts_per_rank, int w
   if (t < T) {
 #pragma unroll
     for (int k = 0; k < TOP_K; ++k) {
-      const int d = __ldg(topk_idx + static_cast<size_t>(t) * TOP_K + k) / experts_per_rank;
+      const int d = ld_dep(topk_idx + static_cast<size_t>(t) * TOP_K + k) / experts_per_rank;
 #pragma unroll
       for (int i = 0; i < E_GLOBAL / 32; ++i)
         if (i == (d >> 5)) mask[i] |= 1u << (d & 31);
@@ -59,10 +59,10 @@ k_dest_bits(const int* __restrict__ topk_idx, int T, int experts_per_rank, int w
 // Record index of every (token, destination) pair: segment start of the destination + rank of the token inside it.
 // slot_map[t,k] gets the index for the FIRST of the token's experts that lives on that destination, -1 for the others.
 __global__ void __launch_bounds__(128)
-k_dispatch_slots(const int* __restrict__ topk_idx, const uint32_t* __restrict__ chunk_bits,
-                 const int* __restrict__ chunk_base, const int* __restrict__ counts, int T, int experts_per_rank,
-                 int world, int n_chunks, int* __restrict__ send_counts, int* __restrict__ slot_token,
-                 int* __restrict__ slot_map) {
+k_dispatch_slots(const int* topk_idx, const uint32_t* chunk_bits,
+                 const int* chunk_base, const int* counts, int T, int experts_per_rank,
+                 int world, int n_chunks, int* send_counts, int* slot_token,
+                 int* slot_map) {
   __shared__ int s_seg[E_GLOBAL + 1];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -73,7 +73,7 @@ k_dispatch_slots(const int* __restrict__ topk_idx, const uint32_t* __restrict__ 
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int d = lane * 8 + i;
-      c[i] = (d < world) ? __ldg(counts + d) : 0;
+      c[i] = (d < world) ? ld_dep(counts + d) : 0;
       local += c[i];
     }
     int incl = local;
@@ -92,7 +92,7 @@ k_dispatch_slots(const int* __restrict__ topk_idx, const uint32_t* __restrict__ 
   }
   __syncthreads();
   if (blockIdx.x == 0)
-    for (int d = threadIdx.x; d < world; d += blockDim.x) send_counts[d] = __ldg(counts + d);
+    for (int d = threadIdx.x; d < world; d += blockDim.x) send_counts[d] = ld_dep(counts + d);
 
   const int chunk = blockIdx.x * (blockDim.x >> 5) + warp;
   if (chunk >= n_chunks) return;
@@ -101,20 +101,23 @@ k_dispatch_slots(const int* __restrict__ topk_idx, const uint32_t* __restrict__ 
   const uint32_t below = (1u << lane) - 1u;
   int dest[TOP_K], slot[TOP_K];
 #pragma unroll
+  for (int k = 0; k < TOP_K; ++k) dest[k] = ld_dep(topk_idx + static_cast<size_t>(t) * TOP_K + k) / experts_per_rank;
+#pragma unroll
   for (int k = 0; k < TOP_K; ++k) {
-    dest[k] = __ldg(topk_idx + static_cast<size_t>(t) * TOP_K + k) / experts_per_rank;
     bool first = true;
 #pragma unroll
     for (int j = 0; j < k; ++j) first = first && (dest[j] != dest[k]);
     slot[k] = -1;
     if (first) {
       const int d = dest[k];
-      const uint32_t bits = __ldg(chunk_bits + static_cast<size_t>(chunk) * world + d);
-      const int s = s_seg[d] + __ldg(chunk_base + static_cast<size_t>(chunk) * world + d) + __popc(bits & below);
+      const uint32_t bits = ld_dep(chunk_bits + static_cast<size_t>(chunk) * world + d);
+      const int s = s_seg[d] + ld_dep(chunk_base + static_cast<size_t>(chunk) * world + d) + __popc(bits & below);
       slot[k] = s;
-      slot_token[s] = t;
     }
   }
+#pragma unroll
+  for (int k = 0; k < TOP_K; ++k)
+    if (slot[k] >= 0) slot_token[slot[k]] = t;
   int4* out = reinterpret_cast<int4*>(slot_map + static_cast<size_t>(t) * TOP_K);
   out[0] = make_int4(slot[0], slot[1], slot[2], slot[3]);
   out[1] = make_int4(slot[4], slot[5], slot[6], slot[7]);
@@ -130,31 +133,31 @@ struct PeerTargets {
 // One warp per record.  With send_rows the records form one local buffer in slot order; with send_rows == nullptr
 // (world <= 8) each record is stored into its destination rank's receive buffer, which may be another GPU's memory.
 __global__ void __launch_bounds__(256)
-k_pack_records(const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale,
-               const int* __restrict__ topk_idx, const float* __restrict__ topk_w, int T, const int* __restrict__ counts,
-               int world, const int* __restrict__ slot_token, uint8_t* __restrict__ send_rows, const PeerTargets peers,
-               const b200moe_ep_plan* __restrict__ plan, int cap_recv, int* __restrict__ check) {
+k_pack_records(const uint8_t* hidden, const float* hidden_scale,
+               const int* topk_idx, const float* topk_w, int T, const int* counts,
+               int world, const int* slot_token, uint8_t* send_rows, const PeerTargets peers,
+               const b200moe_ep_plan* plan, int cap_recv, int* check) {
   const int lane = threadIdx.x & 31;
   const int warps_per_cta = blockDim.x >> 5;
   pdl_launch_dependents();
   pdl_wait();
-  if (plan && !plan->ok) return;   // the counts did not fit the buffers (or the exchange timed out): store nothing
+  if (plan && !ld_l2(&plan->ok)) return;   // the counts did not fit the buffers (or the exchange timed out): store nothing
   int total = 0;
   int seg[9];
 #pragma unroll
   for (int d = 0; d < 8; ++d) {
     seg[d] = total;
-    if (d < world) total += __ldg(counts + d);
+    if (d < world) total += ld_dep(counts + d);
   }
   seg[8] = total;
   if (world > 8)
-    for (int d = 8; d < world; ++d) total += __ldg(counts + d);
+    for (int d = 8; d < world; ++d) total += ld_dep(counts + d);
   // Peer stores: every rank starts with the records for the NEXT rank and wraps around.  In destination order all ranks
   // would write to rank 0 first, then all to rank 1, ...: one receiver's NVLink ingress shared by every sender.
-  const int rot = (plan && !send_rows) ? seg[(plan->rank + 1) % world] : 0;
+  const int rot = (plan && !send_rows) ? seg[(ld_l2(&plan->rank) + 1) % world] : 0;
   for (int s0 = blockIdx.x * warps_per_cta + (threadIdx.x >> 5); s0 < total; s0 += gridDim.x * warps_per_cta) {
     const int s = (s0 + rot < total) ? s0 + rot : s0 + rot - total;
-    const int tok = __ldg(slot_token + s);
+    const int tok = ld_dep(slot_token + s);
     uint8_t* rec;
     if (send_rows) {
       rec = send_rows + static_cast<size_t>(s) * EP_RECORD;
@@ -163,7 +166,7 @@ k_pack_records(const uint8_t* __restrict__ hidden, const float* __restrict__ hid
 #pragma unroll
       for (int j = 1; j < 8; ++j)
         if (s >= seg[j]) d = j;
-      const int row0 = plan ? plan->dst_row0[d] : peers.row0[d];
+      const int row0 = plan ? ld_l2(&plan->dst_row0[d]) : peers.row0[d];
       rec = peers.base[d] + static_cast<size_t>(row0 + (s - seg[d])) * EP_RECORD;
       if (check && ((reinterpret_cast<uintptr_t>(rec) & 15u) || row0 < 0 || row0 + (s - seg[d]) >= cap_recv)) {
         // never store through an address that does not add up: record it and skip the record
@@ -175,16 +178,21 @@ k_pack_records(const uint8_t* __restrict__ hidden, const float* __restrict__ hid
         continue;
       }
     }
-    const uint4* src = reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(tok) * H);
-    uint4* dst = reinterpret_cast<uint4*>(rec);
+    // scales, ids and weights first: their round trip overlaps the row's
+    float scales[2];
 #pragma unroll
-    for (int i = 0; i < H / 16 / 32; ++i) dst[i * 32 + lane] = __ldg(src + i * 32 + lane);
+    for (int i = 0; i < 2; ++i)
+      scales[i] = i * 32 + lane < H_BLOCKS ? ld_dep(hidden_scale + static_cast<size_t>(i * 32 + lane) * T + tok) : 0.f;
+    const int id = lane < TOP_K ? ld_dep(topk_idx + static_cast<size_t>(tok) * TOP_K + lane) : 0;
+    const float w = lane < TOP_K ? ld_dep(topk_w + static_cast<size_t>(tok) * TOP_K + lane) : 0.f;
+    copy_row(rec, hidden + static_cast<size_t>(tok) * H, lane);
     float* sc = reinterpret_cast<float*>(rec + H);
-    for (int kb = lane; kb < H_BLOCKS; kb += 32) sc[kb] = __ldg(hidden_scale + static_cast<size_t>(kb) * T + tok);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (i * 32 + lane < H_BLOCKS) sc[i * 32 + lane] = scales[i];
     if (lane < TOP_K) {
-      reinterpret_cast<int*>(rec + H + 4 * H_BLOCKS)[lane] = __ldg(topk_idx + static_cast<size_t>(tok) * TOP_K + lane);
-      reinterpret_cast<float*>(rec + H + 4 * H_BLOCKS + 4 * TOP_K)[lane] =
-          __ldg(topk_w + static_cast<size_t>(tok) * TOP_K + lane);
+      reinterpret_cast<int*>(rec + H + 4 * H_BLOCKS)[lane] = id;
+      reinterpret_cast<float*>(rec + H + 4 * H_BLOCKS + 4 * TOP_K)[lane] = w;
     }
   }
   if (!send_rows) __threadfence_system();  // peer stores are visible system-wide before the barrier that follows
@@ -197,7 +205,7 @@ static long long g_wait_limit_cycles = WAIT_LIMIT_CYCLES;   // host side: limit 
 
 __global__ void __launch_bounds__(32)
 k_ep_barrier(const PeerTargets flags /* base[r] = rank r's int flags[world] */, int world, int rank, int epoch,
-             long long limit_cycles, int* __restrict__ status) {
+             long long limit_cycles, int* status) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x;
@@ -232,9 +240,9 @@ struct ExchangeTargets {
   float* back[8];
 };
 __global__ void __launch_bounds__(64)
-k_ep_exchange(const ExchangeTargets tg, const int* __restrict__ send_counts, int world, int rank, int epoch,
+k_ep_exchange(const ExchangeTargets tg, const int* send_counts, int world, int rank, int epoch,
               int cap_recv, int cap_back, int back_row_floats, long long limit_cycles,
-              b200moe_ep_plan* __restrict__ plan, int* __restrict__ status) {
+              b200moe_ep_plan* plan, int* status) {
   __shared__ int s_timeout;
   pdl_launch_dependents();
   pdl_wait();
@@ -243,7 +251,7 @@ k_ep_exchange(const ExchangeTargets tg, const int* __restrict__ send_counts, int
   if (tid < world * world) {
     const int d = tid / world, j = tid - d * world;
     volatile int* remote = reinterpret_cast<volatile int*>(tg.counts[d]) + rank * 8 + j;
-    *remote = __ldg(send_counts + j);
+    *remote = ld_dep(send_counts + j);
   }
   __threadfence_system();
   __syncthreads();

@@ -208,8 +208,8 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // T = 120 / 32 179 -> 173.)
   const bool early = args.early_weights != 0;
   if (!early) pdl_wait();
-  for (int i = threadIdx.x; i <= E; i += GEMM_THREADS) aux->off[i] = __ldg(args.block_offsets + i);
-  for (int i = threadIdx.x; i < E; i += GEMM_THREADS) aux->cnt[i] = __ldg(args.counts + i);
+  for (int i = threadIdx.x; i <= E; i += GEMM_THREADS) aux->off[i] = ld_l2(args.block_offsets + i);
+  for (int i = threadIdx.x; i < E; i += GEMM_THREADS) aux->cnt[i] = ld_l2(args.counts + i);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -354,7 +354,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
       for (int i = 0; i < (C::W_SCALES + 31) / 32; ++i) {
         const int j = i * 32 + lane;
-        if (j < C::W_SCALES) w_next[i] = __ldg(src + j + ((MODE == 1 && j >= H_BLOCKS) ? 15 * H_BLOCKS : 0));
+        if (j < C::W_SCALES) w_next[i] = ld_dep(src + j + ((MODE == 1 && j >= H_BLOCKS) ? 15 * H_BLOCKS : 0));
       }
     };
     auto keep_scales = [&]() {

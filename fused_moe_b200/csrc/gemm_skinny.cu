@@ -166,9 +166,9 @@ __device__ __forceinline__ bool run_item(const GemmArgs& args, Aux* aux, const T
   {
     const float4* nx = reinterpret_cast<const float4*>(xs_ptr + static_cast<size_t>(it.kb0) * args.R_max);
 #pragma unroll
-    for (int v = 0; v < NC / 4; ++v) xs_n[v] = __ldg(nx + v);
+    for (int v = 0; v < NC / 4; ++v) xs_n[v] = ld_dep(nx + v);
   }
-  float w0_n = __ldg(w0_ptr + it.kb0), w1_n = __ldg(w1_ptr + it.kb0);
+  float w0_n = ld_dep(w0_ptr + it.kb0), w1_n = ld_dep(w1_ptr + it.kb0);
 
   for (int kb = it.kb0; kb < it.kb1; ++kb) {
     float xs[NC];
@@ -180,9 +180,9 @@ __device__ __forceinline__ bool run_item(const GemmArgs& args, Aux* aux, const T
     if (kb + 1 < it.kb1) {
       const float4* nx = reinterpret_cast<const float4*>(xs_ptr + static_cast<size_t>(kb + 1) * args.R_max);
 #pragma unroll
-      for (int v = 0; v < NC / 4; ++v) xs_n[v] = __ldg(nx + v);
-      w0_n = __ldg(w0_ptr + kb + 1);
-      w1_n = __ldg(w1_ptr + kb + 1);
+      for (int v = 0; v < NC / 4; ++v) xs_n[v] = ld_dep(nx + v);
+      w0_n = ld_dep(w0_ptr + kb + 1);
+      w1_n = ld_dep(w1_ptr + kb + 1);
     }
     if (!mbar_wait_all(smem_u32(&aux->tfull[ps.acc]), ps.acc_phase, abort_flag, args.status, 4, kb)) return false;
     tc_fence_after();
@@ -242,8 +242,8 @@ __device__ __forceinline__ bool run_item(const GemmArgs& args, Aux* aux, const T
       const float* src = args.partial + static_cast<size_t>(c * 2 + slot) * SLOT_FLOATS + q * 32 + lane;
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
-        const float v0 = __ldcg(src + (col0 + j) * 128);
-        const float v1 = __ldcg(src + (SUB_M + col0 + j) * 128);
+        const float v0 = ld_l2(src + (col0 + j) * 128);
+        const float v1 = ld_l2(src + (SUB_M + col0 + j) * 128);
         a0[j] = (c == c_first) ? v0 : a0[j] + v0;
         a1[j] = (c == c_first) ? v1 : a1[j] + v1;
       }
@@ -344,8 +344,8 @@ k_grouped_gemm_skinny(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   // CTA-local set-up above may overlap the tail of the previous kernel; what that kernel wrote is read from here on
   if (!early) pdl_wait();
   if (MODE == 1 && !early) pdl_launch_dependents();
-  for (int i = threadIdx.x; i <= E; i += THREADS) aux->off[i] = __ldg(args.block_offsets + i);
-  for (int i = threadIdx.x; i < E; i += THREADS) aux->cnt[i] = __ldg(args.counts + i);
+  for (int i = threadIdx.x; i <= E; i += THREADS) aux->off[i] = ld_l2(args.block_offsets + i);
+  for (int i = threadIdx.x; i < E; i += THREADS) aux->cnt[i] = ld_l2(args.counts + i);
   __syncthreads();
   if (warp == 0) {
     // sub-blocks per expert = ceil(count / 64), exclusive prefix over experts; lane handles experts [8*lane, 8*lane+8)

@@ -45,8 +45,8 @@ __device__ __forceinline__ void store_half_group(uint8_t* row, int v, const floa
 }
 // acc += w * (group v of the half row at `row`).  2^(eb - 141) * w is exact (eb = 14 decodes to zero).
 __device__ __forceinline__ void fma_half_group(const uint8_t* row, int v, float w, float (&acc)[8]) {
-  const uint4 q = __ldg(reinterpret_cast<const uint4*>(row) + v);
-  const uint32_t eb = __ldg(row + HALF_ROW_SCALES + v);
+  const uint4 q = ld_dep(reinterpret_cast<const uint4*>(row) + v);
+  const uint32_t eb = ld_dep(row + HALF_ROW_SCALES + v);
   const float k = __uint_as_float((eb - 14u) << 23) * w;
   const uint32_t x[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll

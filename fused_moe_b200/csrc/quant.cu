@@ -18,7 +18,7 @@ __device__ __forceinline__ uint32_t quantize_pair(float a, float b, float inv) {
 }
 
 __global__ void __launch_bounds__(256)
-k_quantize_act(const uint4* __restrict__ x, int T, uint2* __restrict__ q, float* __restrict__ scale) {
+k_quantize_act(const uint4* x, int T, uint2* q, float* scale) {
   const int lane = threadIdx.x & 31;
   const int sub = lane & 15;        // lane within the half-warp that owns one 128-column block
   const uint32_t half_mask = (lane & 16) ? 0xffff0000u : 0x0000ffffu;
@@ -33,7 +33,7 @@ k_quantize_act(const uint4* __restrict__ x, int T, uint2* __restrict__ q, float*
 #pragma unroll
     for (int i = 0; i < UNROLL; ++i) {
       const long long p = p0 + i * half_warps;
-      raw[i] = p < total ? __ldg(x + p * 16 + sub) : make_uint4(0u, 0u, 0u, 0u);   // 8 bf16
+      raw[i] = p < total ? ld_dep(x + p * 16 + sub) : make_uint4(0u, 0u, 0u, 0u);   // 8 bf16
     }
 #pragma unroll
     for (int i = 0; i < UNROLL; ++i) {

@@ -39,14 +39,14 @@ __device__ __forceinline__ float key2f(uint32_t k) {
 
 // Routing of one token by one warp.  Lane k < 8 returns the k-th selected expert in `my_idx` and its final weight in
 // `my_w` (other lanes return 0).
-__device__ __forceinline__ void route_token(const float* __restrict__ logits_row, const uint16_t* __restrict__ bias,
+__device__ __forceinline__ void route_token(const float* logits_row, const uint16_t* bias,
                                             float scale_factor, int lane, int& my_idx, float& my_w) {
   float s[N_GROUP];
   uint32_t key[N_GROUP];
 #pragma unroll
   for (int g = 0; g < N_GROUP; ++g) {
-    float x = __ldg(logits_row + g * 32 + lane);
-    float b = bf16_bits_to_float(__ldg(bias + g * 32 + lane));
+    float x = ld_dep(logits_row + g * 32 + lane);
+    float b = bf16_bits_to_float(ld_dep(bias + g * 32 + lane));
     s[g] = sigmoid_exact_ops(x);
     key[g] = f2key(__fadd_rn(s[g], b));
   }

@@ -24,9 +24,9 @@ namespace b200moe {
 // (4 CTAs each), so every byte of every mask word is written even where the last chunk is ragged.
 constexpr int ROUTE_WARPS = 8;
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
-k_route(const float* __restrict__ logits, const uint16_t* __restrict__ bias, int T, float scale_factor,
-        int local_offset, int E_local, int* __restrict__ topk_idx, float* __restrict__ topk_w,
-        uint32_t* __restrict__ chunk_bits) {
+k_route(const float* logits, const uint16_t* bias, int T, float scale_factor,
+        int local_offset, int E_local, int* topk_idx, float* topk_w,
+        uint32_t* chunk_bits) {
   __shared__ uint32_t s_bits[E_GLOBAL];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -67,12 +67,12 @@ k_route(const float* __restrict__ logits, const uint16_t* __restrict__ bias, int
 constexpr int SMALL_T_MAX = B200MOE_PROLOGUE_MAX_T;
 static_assert(SMALL_T_MAX % 32 == 0 && SMALL_T_MAX <= 128, "whole token chunks, at most 1024 (token, k) pairs");
 __global__ void __launch_bounds__(1024, 1)
-k_small_prologue(const float* __restrict__ logits, const uint16_t* __restrict__ bias, const uint8_t* __restrict__ hidden,
-                 const float* __restrict__ hidden_scale, int T, float scale_factor, int local_offset, int E_local,
-                 int R_max, int* __restrict__ topk_idx, float* __restrict__ topk_w, uint32_t* __restrict__ chunk_bits,
-                 int* __restrict__ chunk_base, int* __restrict__ counts, int* __restrict__ block_offsets,
-                 int* __restrict__ total_blocks, int* __restrict__ sorted_token_ids, float* __restrict__ sorted_weights,
-                 int* __restrict__ scatter_map, uint8_t* __restrict__ a_sorted, float* __restrict__ a_scale_sorted) {
+k_small_prologue(const float* logits, const uint16_t* bias, const uint8_t* hidden,
+                 const float* hidden_scale, int T, float scale_factor, int local_offset, int E_local,
+                 int R_max, int* topk_idx, float* topk_w, uint32_t* chunk_bits,
+                 int* chunk_base, int* counts, int* block_offsets,
+                 int* total_blocks, int* sorted_token_ids, float* sorted_weights,
+                 int* scatter_map, uint8_t* a_sorted, float* a_scale_sorted) {
   __shared__ uint32_t s_bits[SMALL_T_MAX / 32][E_GLOBAL];
   __shared__ int s_base[SMALL_T_MAX / 32][E_GLOBAL];
   __shared__ int s_cnt[E_GLOBAL];
@@ -185,25 +185,22 @@ k_small_prologue(const float* __restrict__ logits, const uint16_t* __restrict__ 
     const int d = s_dest[pair];
     if (d < 0) continue;
     const int tok = pair / TOP_K;
-    const uint4* src = reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(tok) * H);
-    uint4* dst = reinterpret_cast<uint4*>(a_sorted + static_cast<size_t>(d) * H);
-#pragma unroll
-    for (int i = 0; i < H / 16 / 32; ++i) dst[i * 32 + lane] = __ldg(src + i * 32 + lane);
+    copy_row(a_sorted + static_cast<size_t>(d) * H, hidden + static_cast<size_t>(tok) * H, lane);
     for (int kb = lane; kb < H_BLOCKS; kb += 32)
-      a_scale_sorted[static_cast<size_t>(kb) * R_max + d] = __ldg(hidden_scale + static_cast<size_t>(kb) * T + tok);
+      a_scale_sorted[static_cast<size_t>(kb) * R_max + d] = ld_dep(hidden_scale + static_cast<size_t>(kb) * T + tok);
   }
 }
 
 // chunk_bits from an existing topk_idx: one warp per 32-token chunk, lane = token.
 __global__ void __launch_bounds__(128)
-k_topk_bits(const int* __restrict__ topk_idx, long long idx_stride, int T, int local_offset, int E_local, int n_chunks,
-            uint32_t* __restrict__ chunk_bits, const b200moe_ep_plan* __restrict__ plan) {
+k_topk_bits(const int* topk_idx, long long idx_stride, int T, int local_offset, int E_local, int n_chunks,
+            uint32_t* chunk_bits, const b200moe_ep_plan* plan) {
   const int lane = threadIdx.x & 31;
   const int chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   pdl_launch_dependents();
   pdl_wait();
   if (chunk >= n_chunks) return;
-  if (plan) T = min(T, plan->n_recv);   // rows past the received count hold stale records: they select nothing
+  if (plan) T = min(T, ld_l2(&plan->n_recv));   // rows past the received count hold stale records: they select nothing
   const int t = chunk * 32 + lane;
   uint32_t mask[E_GLOBAL / 32];
 #pragma unroll
@@ -211,7 +208,7 @@ k_topk_bits(const int* __restrict__ topk_idx, long long idx_stride, int T, int l
   if (t < T) {
 #pragma unroll
     for (int k = 0; k < TOP_K; ++k) {
-      int le = __ldg(topk_idx + static_cast<size_t>(t) * idx_stride + k) - local_offset;
+      int le = ld_dep(topk_idx + static_cast<size_t>(t) * idx_stride + k) - local_offset;
       if (le >= 0 && le < E_local) {
 #pragma unroll
         for (int i = 0; i < E_GLOBAL / 32; ++i)

@@ -22,8 +22,8 @@ namespace b200moe {
 // and writes chunk_base.  (Two earlier layouts, one warp per expert with a lane per chunk or per run of chunks, touched
 // 32 lines per load instruction and took 24 - 30 us at 512 chunks x 256 experts.)
 __global__ void __launch_bounds__(1024)
-k_rank_scan(const uint32_t* __restrict__ chunk_bits, int n_chunks, int E_local, int* __restrict__ chunk_base,
-            int* __restrict__ counts) {
+k_rank_scan(const uint32_t* chunk_bits, int n_chunks, int E_local, int* chunk_base,
+            int* counts) {
   __shared__ int s_run[32][33];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -38,7 +38,7 @@ k_rank_scan(const uint32_t* __restrict__ chunk_bits, int n_chunks, int E_local, 
   int sum = 0;
   if (live) {
 #pragma unroll 8
-    for (int c = c0; c < c1; ++c) sum += __popc(__ldg(col + static_cast<size_t>(c) * E_local));
+    for (int c = c0; c < c1; ++c) sum += __popc(ld_dep(col + static_cast<size_t>(c) * E_local));
   }
   s_run[warp][lane] = sum;
   __syncthreads();
@@ -47,10 +47,16 @@ k_rank_scan(const uint32_t* __restrict__ chunk_bits, int n_chunks, int E_local, 
   if (live) {
     if (warp == 31) counts[e] = run + sum;
     int* out = chunk_base + e;
-#pragma unroll 8
-    for (int c = c0; c < c1; ++c) {
-      out[static_cast<size_t>(c) * E_local] = run;
-      run += __popc(__ldg(col + static_cast<size_t>(c) * E_local));
+    for (int c = c0; c < c1; c += 8) {   // eight words in flight, then their stores
+      uint32_t bits[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) bits[i] = c + i < c1 ? ld_dep(col + static_cast<size_t>(c + i) * E_local) : 0u;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c + i < c1) {
+          out[static_cast<size_t>(c + i) * E_local] = run;
+          run += __popc(bits[i]);
+        }
     }
   }
 }
@@ -62,12 +68,12 @@ k_rank_scan(const uint32_t* __restrict__ chunk_bits, int n_chunks, int E_local, 
 constexpr int SCATTER_SCAN_MAX_CHUNKS = 32;
 template <bool SCAN>
 __global__ void __launch_bounds__(128)
-k_scatter(const int* __restrict__ topk_idx, const float* __restrict__ topk_w, long long topk_stride,
-          const uint32_t* __restrict__ chunk_bits,
-          const int* __restrict__ chunk_base, int* __restrict__ counts, int T, int local_offset, int E_local,
-          int n_chunks, int* __restrict__ block_offsets, int* __restrict__ total_blocks,
-          int* __restrict__ sorted_token_ids, float* __restrict__ sorted_weights, int* __restrict__ scatter_map,
-          const b200moe_ep_plan* __restrict__ plan) {
+k_scatter(const int* topk_idx, const float* topk_w, long long topk_stride,
+          const uint32_t* chunk_bits,
+          const int* chunk_base, int* counts, int T, int local_offset, int E_local,
+          int n_chunks, int* block_offsets, int* total_blocks,
+          int* sorted_token_ids, float* sorted_weights, int* scatter_map,
+          const b200moe_ep_plan* plan) {
   __shared__ int s_row_base[E_GLOBAL + 1];
   __shared__ int s_cnt[SCAN ? E_GLOBAL : 1];
   __shared__ int s_base[SCAN ? 4 : 1][SCAN ? E_GLOBAL : 1];
@@ -83,7 +89,7 @@ k_scatter(const int* __restrict__ topk_idx, const float* __restrict__ topk_w, lo
 #pragma unroll 8
       for (int c = 0; c < n_chunks; ++c) {
         if (c >= c_first && c < c_first + 4) s_base[c - c_first][e] = run;
-        run += __popc(__ldg(chunk_bits + static_cast<size_t>(c) * E_local + e));
+        run += __popc(ld_dep(chunk_bits + static_cast<size_t>(c) * E_local + e));
       }
       s_cnt[e] = run;
       if (blockIdx.x == 0) counts[e] = run;
@@ -97,7 +103,7 @@ k_scatter(const int* __restrict__ topk_idx, const float* __restrict__ topk_w, lo
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       int e = lane * 8 + i;
-      int c = (e < E_local) ? (SCAN ? s_cnt[e] : __ldg(counts + e)) : 0;
+      int c = (e < E_local) ? (SCAN ? s_cnt[e] : ld_dep(counts + e)) : 0;
       blocks[i] = (c + BLOCK_M - 1) / BLOCK_M;
       local += blocks[i];
     }
@@ -127,7 +133,7 @@ k_scatter(const int* __restrict__ topk_idx, const float* __restrict__ topk_w, lo
   // at a time, 40 tokens left one CTA to pad 256 experts one after the other: sort 19.4 us, now 4.6; 113 tokens / 128 experts
   // 12.8 -> 4.7, 2048 / 256 10.2 -> 8.1, 80 / 32 5.9 -> 4.3, 16384 / 256 10.2 -> 10.6.)
   for (int e = blockIdx.x * 4 + warp; e < E_local; e += gridDim.x * 4) {
-    const int begin = s_row_base[e] * BLOCK_M + (SCAN ? s_cnt[e] : __ldg(counts + e));
+    const int begin = s_row_base[e] * BLOCK_M + (SCAN ? s_cnt[e] : ld_dep(counts + e));
     const int end = s_row_base[e + 1] * BLOCK_M;
     for (int r = begin + lane; r < end; r += 32) {
       sorted_token_ids[r] = T;
@@ -139,23 +145,29 @@ k_scatter(const int* __restrict__ topk_idx, const float* __restrict__ topk_w, lo
   if (chunk >= n_chunks) return;
   const int t = chunk * 32 + lane;
   // with a device-side plan only the received rows exist; pad rows keep the id T (the capacity) either way
-  if (t >= (plan ? min(T, plan->n_recv) : T)) return;
+  if (t >= (plan ? min(T, ld_l2(&plan->n_recv)) : T)) return;
   const uint32_t below = (1u << lane) - 1u;
-  int dest[TOP_K];
+  int le[TOP_K], dest[TOP_K];
+  float w[TOP_K];
+  uint32_t bits[TOP_K];
+#pragma unroll
+  for (int k = 0; k < TOP_K; ++k) le[k] = ld_dep(topk_idx + static_cast<size_t>(t) * topk_stride + k) - local_offset;
 #pragma unroll
   for (int k = 0; k < TOP_K; ++k) {
-    int le = __ldg(topk_idx + static_cast<size_t>(t) * topk_stride + k) - local_offset;
     dest[k] = -1;
-    if (le >= 0 && le < E_local) {
-      uint32_t bits = __ldg(chunk_bits + static_cast<size_t>(chunk) * E_local + le);
-      int rank = (SCAN ? s_base[warp][le] : __ldg(chunk_base + static_cast<size_t>(chunk) * E_local + le)) +
-                 __popc(bits & below);
-      int d = s_row_base[le] * BLOCK_M + rank;
-      dest[k] = d;
-      sorted_token_ids[d] = t;
-      sorted_weights[d] = __ldg(topk_w + static_cast<size_t>(t) * topk_stride + k);
+    if (le[k] >= 0 && le[k] < E_local) {
+      bits[k] = ld_dep(chunk_bits + static_cast<size_t>(chunk) * E_local + le[k]);
+      dest[k] = SCAN ? s_base[warp][le[k]] : ld_dep(chunk_base + static_cast<size_t>(chunk) * E_local + le[k]);
+      w[k] = ld_dep(topk_w + static_cast<size_t>(t) * topk_stride + k);
     }
   }
+#pragma unroll
+  for (int k = 0; k < TOP_K; ++k)
+    if (dest[k] >= 0) {
+      dest[k] += s_row_base[le[k]] * BLOCK_M + __popc(bits[k] & below);
+      sorted_token_ids[dest[k]] = t;
+      sorted_weights[dest[k]] = w[k];
+    }
   int4* out = reinterpret_cast<int4*>(scatter_map + static_cast<size_t>(t) * TOP_K);
   out[0] = make_int4(dest[0], dest[1], dest[2], dest[3]);
   out[1] = make_int4(dest[4], dest[5], dest[6], dest[7]);
@@ -168,10 +180,10 @@ k_scatter(const int* __restrict__ topk_idx, const float* __restrict__ topk_w, lo
 // 4 bytes at a stride of 4 R_max, the kernel took 345 us for 131072 rows, now 319; 1500 tokens / 64 experts 11.3 -> 9.0 us,
 // 333 tokens / 32 experts 5.2 -> 4.3 us.)
 __global__ void __launch_bounds__(256)
-k_gather(const uint8_t* __restrict__ hidden, long long row_stride, const float* __restrict__ hidden_scale,
+k_gather(const uint8_t* hidden, long long row_stride, const float* hidden_scale,
          long long scale_token_stride, long long scale_block_stride, int T,
-         const int* __restrict__ sorted_token_ids, const int* __restrict__ total_blocks, int R_max, int row_ctas,
-         uint8_t* __restrict__ a_sorted, float* __restrict__ a_scale_sorted) {
+         const int* sorted_token_ids, const int* total_blocks, int R_max, int row_ctas,
+         uint8_t* a_sorted, float* a_scale_sorted) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int warps_per_cta = blockDim.x >> 5;
@@ -180,29 +192,26 @@ k_gather(const uint8_t* __restrict__ hidden, long long row_stride, const float* 
   // weight stages while the rows are still being copied; the roles that read those rows wait for this kernel as usual.
   pdl_wait();
   pdl_launch_dependents();
-  const int rows = __ldg(total_blocks) * BLOCK_M;
+  const int rows = ld_dep(total_blocks) * BLOCK_M;
   if (static_cast<int>(blockIdx.x) >= row_ctas) {
     constexpr int PER = H_BLOCKS / 8;   // scale blocks of a warp: the eight warps of a CTA share 32 rows
     for (int r0 = (blockIdx.x - row_ctas) * 32; r0 < rows; r0 += (gridDim.x - row_ctas) * 32) {
-      const int tok = __ldg(sorted_token_ids + r0 + lane);
+      const int tok = ld_dep(sorted_token_ids + r0 + lane);
       if (tok >= T) continue;
       const float* src = hidden_scale + static_cast<size_t>(tok) * scale_token_stride +
                          static_cast<size_t>(warp * PER) * scale_block_stride;
       float v[PER];
 #pragma unroll
-      for (int i = 0; i < PER; ++i) v[i] = __ldg(src + static_cast<size_t>(i) * scale_block_stride);
+      for (int i = 0; i < PER; ++i) v[i] = ld_dep(src + static_cast<size_t>(i) * scale_block_stride);
 #pragma unroll
       for (int i = 0; i < PER; ++i) a_scale_sorted[static_cast<size_t>(warp * PER + i) * R_max + r0 + lane] = v[i];
     }
     return;
   }
   for (int r = blockIdx.x * warps_per_cta + warp; r < rows; r += row_ctas * warps_per_cta) {
-    const int tok = __ldg(sorted_token_ids + r);
+    const int tok = ld_dep(sorted_token_ids + r);
     if (tok >= T) continue;
-    const uint4* src = reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(tok) * row_stride);
-    uint4* dst = reinterpret_cast<uint4*>(a_sorted + static_cast<size_t>(r) * H);
-#pragma unroll
-    for (int i = 0; i < H / 16 / 32; ++i) dst[i * 32 + lane] = __ldg(src + i * 32 + lane);
+    copy_row(a_sorted + static_cast<size_t>(r) * H, hidden + static_cast<size_t>(tok) * row_stride, lane);
   }
 }
 
@@ -228,9 +237,9 @@ __device__ __forceinline__ int swizzled_slot(int slot) {   // slot = 4 * lane + 
 }
 template <int G>
 __global__ void __launch_bounds__(128)
-k_reduce(const float* __restrict__ expert_out, const int* __restrict__ scatter_map, const float* __restrict__ topk_w,
-         long long w_stride, int T, uint16_t* __restrict__ out, float* __restrict__ out_f32, const OutSegments segs,
-         const b200moe_ep_plan* __restrict__ plan, int* __restrict__ status, int* __restrict__ status_mirror,
+k_reduce(const float* expert_out, const int* scatter_map, const float* topk_w,
+         long long w_stride, int T, uint16_t* out, float* out_f32, const OutSegments segs,
+         const b200moe_ep_plan* plan, int* status, int* status_mirror,
          int half_rows, int half_src) {
   int t = blockIdx.x;
   // un-rounded rows: float32 [7168] or the half form; either way `pitch` floats apart
@@ -252,7 +261,7 @@ k_reduce(const float* __restrict__ expert_out, const int* __restrict__ scatter_m
   pdl_wait();
   // This is the last kernel of a layer call: if an earlier kernel of the call gave up on a wait, copy the status word
   // to the host-visible mirror (plain stores into mapped host memory), where the host sees it without synchronising.
-  if (status_mirror && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && status[0] != 0) {
+  if (status_mirror && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && ld_dep(status) != 0) {
     status_mirror[1] = status[1];
     status_mirror[2] = status[2];
     status_mirror[3] = status[3];
@@ -261,19 +270,24 @@ k_reduce(const float* __restrict__ expert_out, const int* __restrict__ scatter_m
   }
   if (plan) {
     // the row window and the destinations were decided on the device (expert-parallel receiver)
-    const int n = plan->n_recv;
+    const int n = ld_l2(&plan->n_recv), seg_count = ld_l2(&plan->seg_count), next_rank = ld_l2(&plan->rank) + 1;
+    int start[8];   // together with the words above: one round trip
+#pragma unroll
+    for (int j = 0; j < 8; ++j) start[j] = ld_l2(&plan->seg_start[j]);
     if (t >= n) return;
     // CTAs are scheduled in index order and the rows of one sender are contiguous: start with the rows of the NEXT rank
     // and wrap around, so that the ranks return rows to different peers at any moment instead of all to rank 0 first
     // (one receiver's NVLink ingress shared by every sender), then all to rank 1, ...
-    t += plan->seg_start[(plan->rank + 1) % plan->seg_count];
-    if (t >= n) t -= n;
-    int i = 0;
 #pragma unroll
     for (int j = 1; j < 8; ++j)
-      if (j < plan->seg_count && t >= plan->seg_start[j]) i = j;
+      if (j < seg_count && j == next_rank) t += start[j];   // rank 0 starts at row 0
+    if (t >= n) t -= n;
+    int i = 0, first = 0;
+#pragma unroll
+    for (int j = 1; j < 8; ++j)
+      if (j < seg_count && t >= start[j]) { i = j; first = start[j]; }
     out = nullptr;
-    dst_row = plan->seg_base[i] + static_cast<size_t>(t - plan->seg_start[i]) * pitch;
+    dst_row = ld_l2(&plan->seg_base[i]) + static_cast<size_t>(t - first) * pitch;
     if (reinterpret_cast<uintptr_t>(dst_row) & 15u) {
       // never store through an address that does not add up: record it (status code 4) and skip the row
       if (status && threadIdx.x == 0 && atomicCAS(status, 0, 4) == 0) {
@@ -285,8 +299,8 @@ k_reduce(const float* __restrict__ expert_out, const int* __restrict__ scatter_m
     }
   }
   if (threadIdx.x < TOP_K) {
-    s_pos[threadIdx.x] = __ldg(scatter_map + static_cast<size_t>(t) * TOP_K + threadIdx.x);
-    s_w[threadIdx.x] = topk_w ? __ldg(topk_w + static_cast<size_t>(t) * w_stride + threadIdx.x) : 1.0f;
+    s_pos[threadIdx.x] = ld_dep(scatter_map + static_cast<size_t>(t) * TOP_K + threadIdx.x);
+    s_w[threadIdx.x] = topk_w ? ld_dep(topk_w + static_cast<size_t>(t) * w_stride + threadIdx.x) : 1.0f;
   }
   __syncthreads();
   // gridDim.y CTAs share a token's 896 eight-column vectors (small batches: a token per CTA left most SMs idle and
@@ -306,10 +320,10 @@ k_reduce(const float* __restrict__ expert_out, const int* __restrict__ scatter_m
       if (G > 1) {
         // half-form source rows, four groups per thread (only launched with half_src)
         const uint8_t* row = reinterpret_cast<const uint8_t*>(expert_out) + static_cast<size_t>(pos) * HALF_ROW_BYTES;
-        const uint32_t sc4 = __ldg(reinterpret_cast<const uint32_t*>(row + HALF_ROW_SCALES) + u);
+        const uint32_t sc4 = ld_dep(reinterpret_cast<const uint32_t*>(row + HALF_ROW_SCALES) + u);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-          const uint4 q = __ldg(reinterpret_cast<const uint4*>(row) + G * u + g);
+          const uint4 q = ld_dep(reinterpret_cast<const uint4*>(row) + G * u + g);
           const float kw = __uint_as_float((((sc4 >> (8 * g)) & 0xffu) - 14u) << 23) * w;
           const uint32_t x[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -327,7 +341,7 @@ k_reduce(const float* __restrict__ expert_out, const int* __restrict__ scatter_m
         continue;
       }
       const float4* src = reinterpret_cast<const float4*>(expert_out + static_cast<size_t>(pos) * H) + 2 * u;
-      float4 a = __ldg(src), b = __ldg(src + 1);
+      float4 a = ld_dep(src), b = ld_dep(src + 1);
       acc[0][0] = fmaf(w, a.x, acc[0][0]); acc[0][1] = fmaf(w, a.y, acc[0][1]);
       acc[0][2] = fmaf(w, a.z, acc[0][2]); acc[0][3] = fmaf(w, a.w, acc[0][3]);
       acc[0][4] = fmaf(w, b.x, acc[0][4]); acc[0][5] = fmaf(w, b.y, acc[0][5]);
@@ -381,12 +395,12 @@ k_reduce(const float* __restrict__ expert_out, const int* __restrict__ scatter_m
 // partial rows travelled in the half form.  Same work split as k_reduce (G groups of eight columns per thread).
 template <int G>
 __global__ void __launch_bounds__(128)
-k_combine_half(const uint8_t* __restrict__ rows, const int* __restrict__ slot_map, int T, uint16_t* __restrict__ out) {
+k_combine_half(const uint8_t* rows, const int* slot_map, int T, uint16_t* out) {
   const int t = blockIdx.x;
   __shared__ int s_pos[TOP_K];
   pdl_launch_dependents();
   pdl_wait();
-  if (threadIdx.x < TOP_K) s_pos[threadIdx.x] = __ldg(slot_map + static_cast<size_t>(t) * TOP_K + threadIdx.x);
+  if (threadIdx.x < TOP_K) s_pos[threadIdx.x] = ld_dep(slot_map + static_cast<size_t>(t) * TOP_K + threadIdx.x);
   __syncthreads();
   const int per = (H / 8 / G) / gridDim.y;
   for (int u = blockIdx.y * per + threadIdx.x; u < (blockIdx.y + 1) * per; u += blockDim.x) {
@@ -405,10 +419,10 @@ k_combine_half(const uint8_t* __restrict__ rows, const int* __restrict__ slot_ma
         continue;
       }
       // four adjacent groups per thread: 64 contiguous bytes and one word of scale bytes (see k_reduce)
-      const uint32_t sc4 = __ldg(reinterpret_cast<const uint32_t*>(row + HALF_ROW_SCALES) + u);
+      const uint32_t sc4 = ld_dep(reinterpret_cast<const uint32_t*>(row + HALF_ROW_SCALES) + u);
 #pragma unroll
       for (int g = 0; g < G; ++g) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(row) + G * u + g);
+        const uint4 q = ld_dep(reinterpret_cast<const uint4*>(row) + G * u + g);
         const float kw = __uint_as_float((((sc4 >> (8 * g)) & 0xffu) - 14u) << 23);
         const uint32_t x[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
