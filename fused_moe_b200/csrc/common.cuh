@@ -296,17 +296,23 @@ __device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t a_desc, uint
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// The same, naming the loaded registers: what uses them cannot be scheduled above the wait.
-#define B200MOE_RW8(r, i) "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7])
-__device__ __forceinline__ void tc_wait_ld(uint32_t (&a)[32], uint32_t (&b)[32]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : B200MOE_RW8(a, 0), B200MOE_RW8(a, 8), B200MOE_RW8(a, 16), B200MOE_RW8(a, 24),
-                 B200MOE_RW8(b, 0), B200MOE_RW8(b, 8), B200MOE_RW8(b, 16), B200MOE_RW8(b, 24)
-               :
-               : "memory");
+// Wait for the warp's tcgen05.ld in flight and name the registers they fill.  The loads return before their registers are
+// valid, a "memory" clobber does not order what uses a register, and an empty statement that "changes" each of them does: no
+// use can be scheduled above the wait.
+template <int N, int M>
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&a)[N], uint32_t (&b)[M]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < N; ++j) asm volatile("" : "+r"(a[j]));
+#pragma unroll
+  for (int j = 0; j < M; ++j) asm volatile("" : "+r"(b[j]));
 }
-#undef B200MOE_RW8
+template <int N>
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&a)[N]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < N; ++j) asm volatile("" : "+r"(a[j]));
+}
 
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp receives lane (base+i), r[j] = column (col0+j).
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {

@@ -424,7 +424,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const float sc = run == 1 ? sc1 : sc0;
           uint32_t tmp[64];
           tmem_ld64(taddr + col, tmp);
-          tc_wait_ld();
+          tc_wait_ld(tmp);
           if (run == 1) {
             // all of this warp's reads of the stage are complete (tcgen05.wait::ld is warp-synchronous): hand it back
             // to the MMA issuer

@@ -191,7 +191,7 @@ __device__ __forceinline__ bool run_item(const GemmArgs& args, Aux* aux, const T
     uint32_t t0[NC], t1[NC];
     tmem_ld_cols<NC>(taddr, t0);
     tmem_ld_cols<NC>(taddr + 128, t1);
-    tc_wait_ld();
+    tc_wait_ld(t0, t1);
     // this warp's reads of the stage are complete: hand it back to the MMA issuer
     tc_fence_before();
     __syncwarp();
