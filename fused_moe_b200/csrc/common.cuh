@@ -133,12 +133,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
-// A shared-memory counter as a one-way signal: the writers add to it, one reader polls it with acquire
-// loads until it reaches `target` (bounded like mbar_wait).  A poll is a plain shared-memory load: nothing parks, and
-// the reader sees the last addition a few tens of cycles after it happens.
-// The addition orders nothing else (see mbar_arrive_relaxed).
-__device__ __forceinline__ void red_add_relaxed_shared(uint32_t* counter, uint32_t v) {
-  asm volatile("red.relaxed.cta.shared::cta.add.u32 [%0], %1;"
+// A shared-memory counter as a one-way signal: the writers add to it with release, one reader polls it with acquire until it
+// reaches `target` (bounded like mbar_wait).  A poll is a plain shared-memory load: nothing parks, and the reader sees the last
+// addition a few tens of cycles after it happens.  A lane that signals for its warp does so behind __syncwarp.
+__device__ __forceinline__ void red_add_release_shared(uint32_t* counter, uint32_t v) {
+  asm volatile("red.release.cta.shared::cta.add.u32 [%0], %1;"
                ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(counter))), "r"(v)
                : "memory");
 }
@@ -175,18 +174,18 @@ __device__ __forceinline__ bool counter_wait(const uint32_t* counter, uint32_t t
   }
 }
 
-// Eight one-byte counters in shared memory as a one-way signal: each of eight writers stores its own running count (modulo
-// 256) with a plain store that orders nothing else (see mbar_arrive_relaxed), one reader polls the word until all of them
-// show `target` (bounded like mbar_wait).  No writer may run past `target` before the reader has seen it.
-__device__ __forceinline__ void st_relaxed_shared_u8(uint8_t* p, uint32_t v) {
-  asm volatile("st.relaxed.cta.shared::cta.u8 [%0], %1;"
+// Eight one-byte counters in shared memory as a one-way signal of the same kind: each of eight writers stores its own running
+// count (modulo 256) with release, one reader polls the word with acquire until all of them show `target` (bounded like
+// mbar_wait).  No writer may run past `target` before the reader has seen it.
+__device__ __forceinline__ void st_release_shared_u8(uint8_t* p, uint32_t v) {
+  asm volatile("st.release.cta.shared::cta.u8 [%0], %1;"
                ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(v)
                : "memory");
 }
 __device__ __forceinline__ bool flags_equal(uint32_t flags8, uint32_t target4) {
-  uint32_t a, b;
-  asm volatile("ld.volatile.shared::cta.v2.u32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(flags8) : "memory");
-  return ((a ^ target4) | (b ^ target4)) == 0;
+  uint64_t v;
+  asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(flags8) : "memory");
+  return ((static_cast<uint32_t>(v) ^ target4) | (static_cast<uint32_t>(v >> 32) ^ target4)) == 0;
 }
 __device__ __forceinline__ bool flags_wait(const uint8_t* flags, uint32_t target, volatile int* abort_flag, int* status,
                                            int role, int detail) {

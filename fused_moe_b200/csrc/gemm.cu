@@ -75,6 +75,7 @@ struct Cfg {
 };
 constexpr int ROW_SCALE_BYTES = BLOCK_M * 4;   // row scales of one chunk
 constexpr int SCALE_RING = 8;                  // chunks whose row scales are kept, see GemmAux::row_scale
+constexpr int SCALE_DRAIN_POLLS = DRAIN_POLLS / 32;   // milliseconds
 
 struct TileInfo {
   int e, nt, mblk, m_local, cnt;
@@ -117,7 +118,7 @@ __device__ __forceinline__ TileInfo decode_tile_from(int tile, int e0, const int
 struct __align__(16) GemmAux {
   uint64_t full[4];
   uint64_t empty[4];
-  uint64_t tfull[2];
+  uint64_t tfull[4];   // GEMM1, per operand stage: see row_scale (GEMM2 has it in `empty`)
   uint64_t xbar[2];
   uint32_t tmem_base;
   int abort_flag;
@@ -128,9 +129,17 @@ struct __align__(16) GemmAux {
   int off[E_GLOBAL + 1];
   int cnt[E_GLOBAL];
   float amax[2][2][BLOCK_M];
-  // Row scales, brought by the producer with the operand boxes of their chunk and covered by the same barrier.  Chunk c is
-  // requested once the MMAs of chunk c - STAGES are complete, and those were issued after every promotion warp had read
-  // chunk c - STAGES - 2, so STAGES + 2 <= SCALE_RING slots are enough.
+  // Row scales, brought by the producer behind the operand boxes of their chunk.  The copy completes on the barrier that the
+  // promotion warps wait on before they touch the chunk's sums (`tfull`; in GEMM2 `empty`), next to the MMAs' commit: whoever
+  // reads a scale has seen its copy complete.  For that the barrier counts two arrivals, the commit and the producer's with the
+  // bytes to expect, which belongs to the chunk's own phase because the producer has seen the one before complete.
+  // Chunk c is requested once the MMAs of chunk c - STAGES are complete.  Those were issued after the issuer had acquired the
+  // hand-back of chunk c - STAGES - 2, which every promotion warp releases behind its reads of TMEM and of the row scales, so
+  // STAGES + 2 <= SCALE_RING slots are enough.
+  // (Completing on the operands' barrier, which the promotion warps never look at, and handing back without release, took the
+  // same: GEMM1 / GEMM2 us at 333 tokens / 32 experts 96.8 / 72.5, now 96.6 / 71.3; 4096 / 32, hot, 71.3 / 59.0, now 70.8 / 58.9;
+  // 14107 / 32, hot, 1385 / 1048, now 1393 / 1049; 16384 / 256 5192 / 4050, now 5183 / 4048.  Barriers of their own for groups of
+  // four chunks, a look and an arrival per group, cost GEMM1 1 % at full clock and 2-6 % under the power cap.)
   alignas(16) float row_scale[SCALE_RING][BLOCK_M];
   float w_scale[NUM_PROMO_WARPS][2 * H_BLOCKS];   // weight scales of the tile, a copy per promotion warp
   // GEMM2 epilogue: per promotion warp, 32 rows x 16 columns (+4 padding: conflict-free 16-byte accesses) through which
@@ -185,12 +194,10 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (warp == PRODUCER_WARP && lane == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(smem_u32(&aux->full[s]), 1);
-      mbar_init(smem_u32(&aux->empty[s]), 1);
+      mbar_init(smem_u32(&aux->empty[s]), MODE == 1 ? 1 : 2);
+      mbar_init(smem_u32(&aux->tfull[s]), 2);
     }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(smem_u32(&aux->tfull[a]), 1);
-      mbar_init(smem_u32(&aux->xbar[a]), NUM_PROMO_WARPS);
-    }
+    for (int a = 0; a < 2; ++a) mbar_init(smem_u32(&aux->xbar[a]), NUM_PROMO_WARPS);
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -228,7 +235,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      long long issued = 0;
+      long long issued = 0, scales_issued = 0;
       bool ok = true;
       auto load_weights = [&](const TileInfo& ti, int kb, uint32_t sB, uint32_t full) {
         if (MODE == 1) {
@@ -244,7 +251,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const TileInfo ti = decode_tile(group_id, aux->off, aux->cnt, E, NT);
           for (; ahead < C::STAGES; ++ahead) {
             const uint32_t full = smem_u32(&aux->full[ahead]);
-            mbar_arrive_expect_tx(full, C::STAGE_BYTES + ROW_SCALE_BYTES);
+            mbar_arrive_expect_tx(full, C::STAGE_BYTES);
             load_weights(ti, ahead, tiles_addr + ahead * C::STAGE_BYTES + C::A_TILES * A_TILE_BYTES, full);
           }
         }
@@ -260,13 +267,19 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const uint32_t sB = sbase + C::A_TILES * A_TILE_BYTES;
           const uint32_t full = smem_u32(&aux->full[stage]);
           const bool requested = issued < ahead;
-          if (!requested) mbar_arrive_expect_tx(full, C::STAGE_BYTES + ROW_SCALE_BYTES);
-          bulk_load(smem_u32(&aux->row_scale[issued % SCALE_RING][0]), rs + static_cast<size_t>(kb) * args.R_max,
-                    ROW_SCALE_BYTES, full);
+          if (!requested) mbar_arrive_expect_tx(full, C::STAGE_BYTES);
           tma_load_2d(sbase, &tmA, full, kb * 128, ti.mblk * BLOCK_M);
           if (MODE == 2) tma_load_2d(sbase + A_TILE_BYTES, &tmA, full, kb * 128, args.R_max + ti.mblk * BLOCK_M);
           if (!requested) load_weights(ti, kb, sB, full);
           ++issued;
+          // (ahead of the operands the copy delays them: GEMM1 71.0 us instead of 70.7 at 4096 / 32, hot)
+          const uint32_t sums = smem_u32(MODE == 1 ? &aux->tfull[stage] : &aux->empty[stage]);
+          if (MODE == 1) ok = mbar_wait(sums, phase ^ 1u, abort_flag, args.status, 9, kb);
+          if (!ok) break;
+          mbar_arrive_expect_tx(sums, ROW_SCALE_BYTES);
+          bulk_load(smem_u32(&aux->row_scale[scales_issued % SCALE_RING][0]), rs + static_cast<size_t>(kb) * args.R_max,
+                    ROW_SCALE_BYTES, sums);
+          ++scales_issued;
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
         }
       }
@@ -278,6 +291,15 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           uint32_t par = static_cast<uint32_t>((n_s - 1) & 1);
           for (int spin = 0; spin < DRAIN_POLLS; ++spin)
             if (mbar_try_wait(smem_u32(&aux->full[s]), par)) break;
+        }
+        // The row scales complete on a barrier that also counts a commit, which may never come: then the polls run out, long
+        // after the copy has landed.
+        for (int s = 0; s < C::STAGES; ++s) {
+          const long long n_s = scales_issued / C::STAGES + ((scales_issued % C::STAGES) > s ? 1 : 0);
+          if (n_s == 0) continue;
+          const uint32_t par = static_cast<uint32_t>((n_s - 1) & 1);
+          for (int spin = 0; spin < SCALE_DRAIN_POLLS; ++spin)
+            if (mbar_try_wait(smem_u32(MODE == 1 ? &aux->tfull[s] : &aux->empty[s]), par)) break;
         }
       }
     }
@@ -319,7 +341,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           // GEMM2's promotion warps wait for `empty` too: one commit (70 cycles of this thread, a second one 130) says both
           // that the operands may be overwritten and that the sums are in TMEM.  Its phase cannot run ahead of a waiter:
           // chunk c + STAGES is issued only after chunk c + STAGES - 2 >= c has left TMEM.
-          if (MODE == 1) tc_commit(smem_u32(&aux->tfull[acc]));
+          if (MODE == 1) tc_commit(smem_u32(&aux->tfull[stage]));
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
           if (MODE == 2) landed = mbar_test(smem_u32(&aux->full[stage]), phase);
           acc ^= 1;
@@ -335,8 +357,6 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int q = warp & 3;       // TMEM lane quarter this warp may read
     const int h = warp >> 2;      // column half
     const int r_in_tile = q * 32 + lane;
-    int acc = 0;
-    uint32_t acc_phase = 0;
     int tile_iter = 0;
     bool ok = true;
     uint32_t chunk = 0;
@@ -399,7 +419,8 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           // this warp has read its part of the stage (tcgen05.wait::ld is warp-synchronous): hand it back, and ask for the
           // next chunk's barrier before folding the rest in
           tc_fence_before();
-          if (lane == 0) st_relaxed_shared_u8(&aux->handed[kb & 1][warp], chunk / 2 + 1);
+          __syncwarp();
+          if (lane == 0) st_release_shared_u8(&aux->handed[kb & 1][warp], chunk / 2 + 1);
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
           const uint32_t next = mbar_test(smem_u32(&aux->empty[stage]), phase);
           fold(acc2 + 32, t2, sc);
@@ -408,12 +429,13 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
       }
       for (int kb = 0; MODE == 1 && kb < C::K_CHUNKS; ++kb) {
-        ok = mbar_wait_all(smem_u32(&aux->tfull[acc]), acc_phase, abort_flag, args.status, 4, kb);
+        ok = mbar_wait_all(smem_u32(&aux->tfull[chunk % C::STAGES]), (chunk / C::STAGES) & 1u, abort_flag, args.status, 4, kb);
         if (!ok) break;
         tc_fence_after();
+        const uint32_t acc = chunk & 1u;
         const float rs = aux->row_scale[chunk % SCALE_RING][r_in_tile];
         const float sc0 = rs * w_own[kb];
-        const float sc1 = rs * w_own[(MODE == 1 ? C::K_CHUNKS : 0) + kb];
+        const float sc1 = rs * w_own[C::W_SCALES - C::K_CHUNKS + kb];
         ++chunk;
         const uint32_t taddr = tmem_base + static_cast<uint32_t>(acc * TILE_N) + (static_cast<uint32_t>(q * 32) << 16);
         // This warp's 128 accumulators are two runs of 64 TMEM columns: [64h, 64h+64) holds W1 ("up") and
@@ -429,7 +451,8 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // all of this warp's reads of the stage are complete (tcgen05.wait::ld is warp-synchronous): hand it back
             // to the MMA issuer
             tc_fence_before();
-            if (lane == 0) red_add_relaxed_shared(&aux->drained[acc], 1u);
+            __syncwarp();
+            if (lane == 0) red_add_release_shared(&aux->drained[acc], 1u);
           }
           const float2 sc2 = make_float2(sc, sc);
 #pragma unroll
@@ -437,8 +460,6 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             acc2[run * 32 + j] = __ffma2_rn(make_float2(__uint_as_float(tmp[2 * j]), __uint_as_float(tmp[2 * j + 1])),
                                             sc2, acc2[run * 32 + j]);
         }
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
       }
       if (!ok) break;
       const TileInfo done = ti;
