@@ -15,28 +15,35 @@
 // row.  MODE 1 uses two 128-row weight boxes per chunk (W1 rows n0.., W3 rows 2048+n0..) laid out back to back so a
 // single N=256 MMA produces both SwiGLU operands; MODE 2 uses one 256-row box of W2 and two A boxes (the two terms).
 //
-// One CTA per tile.  What paces it (cycle stamps, probes): a TMEM stage goes round MMA -> completion signal -> promotion
-// warps read it (two 64-column loads per warp) -> hand-back -> next MMA into it, and with 512 TMEM columns there are
-// only two such stages of 256 columns.  The block scales must not come from global memory in the promotion loop: with
-// loads one chunk ahead (an L2 round trip under load is 600-900 cycles, and a releasing hand-back waits for it as well)
-// that loop was the slowest chain; through shared memory, brought by the producer, GEMM1 went 5212 -> 4915 us at T = 16384 /
-// 256 experts, 1494 -> 1316 at 14107 / 32 (hot experts), 343 -> 312 at 1500 / 64, 110 -> 103 at 333 / 32, GEMM2 unchanged.
+// One CTA per tile.  What paces it: a TMEM stage goes round MMA -> completion signal -> promotion warps read it -> hand-back ->
+// next MMA into it, and with 512 TMEM columns there are only two such stages of 256 columns.  A 128-K chunk, its share of the
+// epilogue included, takes 920-950 cycles in GEMM1 for 512 of tensor work and 1330-1370 in GEMM2 for 1024 (launched back to back
+// for seconds, time x median SM clock under the power cap: T = 16384 / 256 experts 5353 us at 1207 MHz and 4170 at 1140, 14107 /
+// 32 with hot experts 1392 at 1245 and 1072 at 1170, 2048 / 256 1637 at 945 and 1163 at 952).  Pieces, from probes: a look at a
+// barrier ~110 cycles even if it is long complete, a shared-memory atomic 110, a first commit 70, a second 130, a load of 32 / 64
+// TMEM columns with its wait 75 / 156.
+//
+// The block scales must not come from global memory in the promotion loop: with loads one chunk ahead (an L2 round trip under
+// load is 600-900 cycles, and the releasing hand-back waits for it as well) that loop was the slowest chain.  Through shared
+// memory GEMM1 went 5188 -> 4999 and 5056 -> 4836 us (two sessions) at T = 16384 / 256 experts, 1523 -> 1312 and 1475 -> 1295 at
+// 14107 / 32 (hot), 357 -> 332 and 328 -> 323 at 1500 / 64, 99.5 -> 97 at 333 / 32; GEMM2 stayed.
 // GEMM2's loop also spends fewer synchronisations per chunk (one commit, a hand-back byte per warp, barrier looks asked for
-// early, 32-column loads in pairs; a look at a barrier takes ~110 cycles even if it is long complete, a shared-memory
-// atomic 110, a second commit 130): 4225 -> 4122 us at T = 16384 / 256, 1094 -> 1064 at 14107 / 32 (hot experts), 340 -> 332
-// at 4096 / 32 (hot experts), 240 -> 237 at 1500 / 64.  The same in GEMM1 made it 4-7 % SLOWER at T >= 4096, so it keeps its form.
-// A round costs ~600 cycles of tensor work (four MMAs of 128 cycles plus issue
-// gaps) and ~1100-1300 cycles of latencies (barrier wake-ups of 190-280 cycles each way, 260 for the two loads, 150 to
-// the hand-back, 170 to re-check the operands), so two stages keep the tensor pipe ~55 % busy: ~970 cycles per 128-K
-// chunk.  Things that were built, measured and did NOT move it: CTA pairs (tcgen05.mma.cta_group::2, each CTA loading
-// half of the weight tile: fewer L2 bytes, but the hand-back then crosses SMs; 485 vs 456 us, also 7 % of pair padding),
-// a second MMA-issuing thread (one per TMEM stage; with it the issuer has slack and the promotion warps are busy
-// ~850 of every ~980 cycles: wake-up, 64-column load, 32 packed FMAs, load, 32 FMAs, nothing overlapped because 128
-// accumulators + 64 loaded values fill the 232 registers), the last promotion warp issuing the next MMAs itself (the
-// issue of four MMAs blocks its thread for ~430 cycles: 38 % slower), and parking barrier polls with a suspend-time hint.
-// The hand-back itself is a shared-memory counter polled by the
-// issuer (2-7 % faster than an mbarrier).  In isolation the pieces run at 512 (MMA), 320 (promotion, 8 warps) and
-// 610-690 (48 KB of loads per SM from L2, all SMs) cycles per chunk, and ~600 when all three run unsynchronised.
+// early, 32-column loads in pairs): 4225 -> 4122 us at 16384 / 256, 1094 -> 1064 at 14107 / 32 (hot), 240 -> 237 at 1500 / 64.
+// All of these are bursts of 20 ms; whole calls at 16384 / 256, which settle under the power cap, did not get shorter.
+// GEMM1 keeps two commits and the counter: with one commit it took 70.7 instead of 70.0 us at 4096 / 32 (hot, full clock), 1418
+// instead of 1350 at 14107 / 32 (hot), 5338 instead of 5201 at 16384 / 256.  The byte hand-back and the early looks were tried
+// there only together with a test for all-padding warps (4-7 % slower; that test alone costs more), never by themselves.
+//
+// Built and measured on GEMM1 before the scales moved (a chunk then took ~970 cycles), and NOT moving it: CTA pairs
+// (tcgen05.mma.cta_group::2, each CTA loading half of the weight tile: fewer L2 bytes, but the hand-back then crosses SMs; 485
+// vs 456 us, also 7 % of pair padding), a second MMA-issuing thread (one per TMEM stage; the issuer then has slack and the
+// promotion warps are busy ~850 of ~980 cycles, nothing overlapped: 128 sums and 64 loaded values of 232 registers), the last
+// promotion warp issuing the next MMAs itself (the issue of four MMAs blocks its thread for ~430 cycles: 38 % slower), and
+// parking barrier polls with a suspend-time hint.  The hand-back through a shared-memory counter polled by the issuer was 2-7 %
+// faster than an mbarrier.  In isolation the pieces run at 512 (MMA), 320 (promotion, 8 warps) and 610-690 (48 KB of loads per
+// SM from L2, all SMs) cycles per chunk, and ~600 when all three run unsynchronised.
+// Registers (-Xptxas -v): 168 per thread at launch; promotion warps hold 128 sums and 64 (GEMM1) or 96 (GEMM2) loaded values in
+// 232; GEMM1 spills 12 bytes, GEMM2 none.
 //
 // Warp roles (384 threads): warps 0-7 promote TMEM partials into fp32 registers and run the epilogue (warp w owns TMEM
 // lanes 32*(w%4).. and half of the columns), warp 8 issues TMA loads, warp 9 owns TMEM and issues the MMAs, warps 10-11

@@ -177,7 +177,8 @@ k_scatter(const int* topk_idx, const float* topk_w, long long topk_stride,
 // never read).  The first `row_ctas` CTAs copy rows, one warp per row, grid-stride over the rows that exist.  The others
 // copy scales: a warp takes 32 consecutive sorted rows, a lane each, and seven of the 56 scale blocks, so that
 // a_scale_sorted ([block][row]) is written 128 contiguous bytes at a time.  (With the row's own warp writing its 56 scales,
-// 4 bytes at a stride of 4 R_max, the kernel took 345 us for 131072 rows, now 319; 1500 tokens / 64 experts 11.3 -> 9.0 us,
+// 4 bytes at a stride of 4 R_max, the kernel took 345 us for 131072 rows, now 319, and 289
+// with half of a lane's row pieces loaded before the first store; 1500 tokens / 64 experts 11.3 -> 9.0 us,
 // 333 tokens / 32 experts 5.2 -> 4.3 us.)
 __global__ void __launch_bounds__(256)
 k_gather(const uint8_t* hidden, long long row_stride, const float* hidden_scale,
